@@ -436,6 +436,22 @@ def test_device_quantize_pack_is_bit_exact(groupsize):
     check(C, orc.c_gemm(A, q, s, groupsize), "device-packed")
 
 
+@pytest.mark.parametrize("n,k,groupsize", [(256, 128, 128), (256, 128, -1), (768, 1152, 128), (512, 640, -1)])
+def test_device_quantize_pack_edges(n, k, groupsize):
+    """Weights on and one fp16 step beside the rounding boundaries (j + 1/2) * s, far past the clamp, zeros of both signs,
+    scales from the smallest subnormal up; a single group, k ranges that do not fill a block."""
+    rng = np.random.default_rng(n + k)
+    groups = 1 if groupsize == -1 else k // groupsize
+    s = np.exp2(rng.uniform(-24, 6, size=(groups, n))).astype(np.float16)
+    x = rng.integers(-24, 25, size=(n, k)).astype(np.float32) / 2
+    w = (x * np.repeat(s.astype(np.float32).T, k // groups, axis=1)).astype(np.float16)
+    w = (w.view(np.int16) + rng.integers(-1, 2, size=(n, k)) * (w != 0)).astype(np.int16).view(np.float16)
+    B_host, sp_host = pkg.quantize_pack(w, s, groupsize)
+    B_dev, sp_dev = pkg.quantize_pack_device(to_dev(w), to_dev(s), groupsize)
+    assert np.array_equal(B_dev.cpu().numpy(), B_host)
+    assert np.array_equal(sp_dev.cpu().numpy().view(np.uint16), sp_host.view(np.uint16))
+
+
 def test_pair_kernel_dependent_chain_graph_replay():
     """Two large-batch GEMMs (CTA-pair kernel) where the first one's output is the second one's activations,
     eagerly and over CUDA-graph replays; the oracle is evaluated on column windows, fed with the device's own
