@@ -61,6 +61,21 @@ def _load():
 lib = _load()
 
 
+def _load_calls():
+    import torch  # noqa: F401  (brings the libraries that the module links against)
+    try:
+        from . import _torch_calls
+    except ImportError as e:
+        raise ImportError("_torch_calls.so is not built, or for another torch (%s). Build it with "
+                          "`make -C awesome-cute_b200/csrc`." % e) from e
+    _torch_calls.bind(*(ctypes.cast(f, ctypes.c_void_p).value
+                        for f in (lib.w4a16_marlin_gemm, lib.w4a16_quantize_pack_device)))
+    return _torch_calls
+
+
+calls = _load_calls()   # the compiled path from torch tensors to the two entry points above
+
+
 class Plan(ctypes.Structure):
     """w4a16_plan_t of include/w4a16.h"""
     _fields_ = [(n, _i) for n in ("kernel", "tile_rows", "k_per_stage", "workers", "ctas_per_worker", "whole_tile_waves",
