@@ -25,6 +25,7 @@
 #include "w4a16_kernel.cuh"
 #include "w4a16_kernel_2sm.cuh"
 #include "w4a16_kernel_decode.cuh"
+#include "w4a16_kernel_skinny.cuh"
 
 namespace {
 
@@ -190,15 +191,23 @@ struct Maps {
 };
 struct MapKey {
   const void *B, *A, *s, *C;   // C only for the TMA-store epilogue (else null: the maps do not depend on it)
-  int m, n, k, ks, a_rows, grouped;
+  int m, n, k, ks, a_rows, grouped, w_rows;
   bool operator<(const MapKey &o) const {
-    return std::tie(B, A, s, C, m, n, k, ks, a_rows, grouped) < std::tie(o.B, o.A, o.s, o.C, o.m, o.n, o.k, o.ks, o.a_rows, o.grouped);
+    return std::tie(B, A, s, C, m, n, k, ks, a_rows, grouped, w_rows) <
+           std::tie(o.B, o.A, o.s, o.C, o.m, o.n, o.k, o.ks, o.a_rows, o.grouped, o.w_rows);
   }
 };
 std::map<MapKey, Maps> g_maps;   // guarded by g_mu
 
-bool build_maps(const Problem &pr, int ks, int a_rows, bool grouped, bool tma_store, Maps &mp) {
-  {  // weights: int32 [k/16][2n] viewed as [k/16][2n/32][32] so a 128-byte inner box can be swizzled
+// w_rows: the weights as they lie in memory, 256 words (128 columns) x 16-k rows, for the kernel that reads whole words
+bool build_maps(const Problem &pr, int ks, int a_rows, bool grouped, bool tma_store, bool w_rows, Maps &mp) {
+  if (w_rows) {
+    const cuuint64_t dims[2] = {(cuuint64_t)(2 * pr.n), (cuuint64_t)(pr.k / 16)};
+    const cuuint64_t strides[1] = {(cuuint64_t)pr.n * 8};
+    const cuuint32_t box[2] = {256, (cuuint32_t)(ks / 16)};
+    if (!encode(&mp.b, CU_TENSOR_MAP_DATA_TYPE_INT32, 2, pr.B, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_NONE, "B rows"))
+      return false;
+  } else {  // weights: int32 [k/16][2n] viewed as [k/16][2n/32][32] so a 128-byte inner box can be swizzled
     const cuuint64_t dims[3] = {32, (cuuint64_t)(2 * pr.n / 32), (cuuint64_t)(pr.k / 16)};
     const cuuint64_t strides[2] = {128, (cuuint64_t)pr.n * 8};
     const cuuint32_t box[3] = {32, 8, (cuuint32_t)(ks / 16)};
@@ -243,14 +252,14 @@ bool build_maps(const Problem &pr, int ks, int a_rows, bool grouped, bool tma_st
 }
 
 // Takes g_mu for the lookup only.
-bool get_maps(const Problem &pr, int ks, int a_rows, bool grouped, bool tma_store, Maps &out) {
-  if (pr.fixed_partials) return build_maps(pr, ks, a_rows, grouped, tma_store, out);  // the allocation-free entry point keeps nothing, on the host either
-  const MapKey key{pr.B, pr.A, pr.s, tma_store ? pr.C : nullptr, pr.m, pr.n, pr.k, ks, a_rows, grouped ? 1 : 0};
+bool get_maps(const Problem &pr, int ks, int a_rows, bool grouped, bool tma_store, Maps &out, bool w_rows = false) {
+  if (pr.fixed_partials) return build_maps(pr, ks, a_rows, grouped, tma_store, w_rows, out);  // the allocation-free entry point keeps nothing, on the host either
+  const MapKey key{pr.B, pr.A, pr.s, tma_store ? pr.C : nullptr, pr.m, pr.n, pr.k, ks, a_rows, grouped ? 1 : 0, w_rows ? 1 : 0};
   std::lock_guard<std::mutex> lock(g_mu);
   auto it = g_maps.find(key);
   if (it == g_maps.end()) {
     Maps mp;
-    if (!build_maps(pr, ks, a_rows, grouped, tma_store, mp)) return false;
+    if (!build_maps(pr, ks, a_rows, grouped, tma_store, w_rows, mp)) return false;
     if (g_maps.size() >= 1024) g_maps.clear();
     it = g_maps.emplace(key, mp).first;
   }
@@ -507,7 +516,8 @@ int launch_decode_cluster(const Problem &pr) {
 
 // W4A16_TMA_STORE=0 / 1 in the environment picks how finished tiles of the plain GEMM reach C: 2-byte stores from
 // registers, or staged in shared memory and stored by the copy engine (cp.async.bulk.tensor).  Both are compiled
-// and tested; the default is the one measured faster (see tma_store_default).
+// and tested; the default is the one measured faster (see tma_store_default).  The kernel for up to 8 rows has one form: a warp
+// stores 256 contiguous bytes.
 const int g_tma_store = [] {
   const char *e = std::getenv("W4A16_TMA_STORE");
   return (e && (e[0] == '0' || e[0] == '1')) ? e[0] - '0' : -1;
@@ -530,6 +540,100 @@ int launch_decode_cluster_o(const Problem &pr, int cl) {
 }
 int launch_decode_cluster_g(const Problem &pr, int cl) {
   return use_tma_store(pr) ? launch_decode_cluster_o<w4a16::OUT_TMA>(pr, cl) : launch_decode_cluster_o<w4a16::OUT_PLAIN>(pr, cl);
+}
+
+// ---- up to 8 rows on CTAs of half an SM: see w4a16_kernel_skinny.cuh
+// W4A16_SKINNY=0 in the environment keeps these batches on the other kernels (debugging aid, A/B timing)
+const bool g_use_skinny = [] {
+  const char *e = std::getenv("W4A16_SKINNY");
+  return !(e && e[0] == '0');
+}();
+
+// Returns -2 when the kernel does not serve the call.
+template <int KS, bool GROUPED>
+int launch_skinny(const Problem &pr) {
+  using Cfg = w4a16::SkinnyConfig<KS>;
+  auto kern = w4a16::w4a16_skinny_kernel<KS, GROUPED>;
+  static bool attr_done[64] = {false};
+  static int fit[64][9];                 // clusters of 4, 8 CTAs that can be resident together
+  const int nsm = problem_sm_count(pr);
+  if (nsm <= 0) return W4A16_ERR_CUDA;
+
+  cudaLaunchConfig_t cfg = {};
+  cfg.blockDim = dim3((unsigned)Cfg::THREADS);
+  cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
+  cfg.stream = pr.stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = g_use_pdl ? 1 : 0;
+  cfg.attrs = attr;
+  if (!pr.plan) {
+    std::lock_guard<std::mutex> lock(g_mu);
+    if (!attr_done[pr.dev]) {
+      if (!cuda_ok(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES), "cudaFuncSetAttribute") ||
+          !cuda_ok(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100), "cudaFuncSetAttribute"))
+        return W4A16_ERR_CUDA;
+      cfg.numAttrs = 1;
+      for (int cl = 4; cl <= 8; cl *= 2) {
+        attr[0].val.clusterDim.x = (unsigned)cl;
+        cfg.gridDim = dim3((unsigned)(nsm / cl * cl));
+        if (!cuda_ok(cudaOccupancyMaxActiveClusters(&fit[pr.dev][cl], kern, &cfg), "cudaOccupancyMaxActiveClusters")) return W4A16_ERR_CUDA;
+      }
+      attr_done[pr.dev] = true;
+    }
+  }
+  w4a16::Params p{};
+  p.m = pr.m, p.n = pr.n, p.k = pr.k;
+  p.n_tiles = pr.n / w4a16::TILE_N;
+  p.m_tiles = 1;
+  p.k_iters = pr.k / KS;
+  const long total = (long)p.n_tiles * p.k_iters;
+  if (total > 0x7fffffffL) return W4A16_ERR_ARG;
+  p.total_iters = (int)total;
+  p.s = static_cast<const __half *>(pr.s);
+  set_output(p, pr);
+  p.wait_ns = pr.wait_ns;
+
+  // Few tiles: one cluster per tile, as large as fits (two CTAs per SM), while a rank keeps at most 12 stages of 256 k;
+  // deeper, the latency that a cluster saves is less than what idle SMs cost (m = 1, us: 4096 x 4096 4.8 on clusters of 8,
+  // 5.2 on stream-K; 8192 x 8192 8.8 / 9.3; 1024 x 8192 4.3 / 5.4; 8192 x 28672, 28 stages a rank, 23.2 / 22.4;
+  // 1024 x 28672, 14 stages a rank, 9.9 / 9.1).
+  int cl = 1;
+  if (g_use_cluster)
+    for (int c = 4; c <= 8; c *= 2)
+      if (p.n_tiles * c <= 2 * nsm && p.k_iters >= c && p.k_iters * KS <= 12 * 256 * c && (pr.plan || fit[pr.dev][c] >= p.n_tiles)) cl = c;
+  int grid = p.n_tiles * cl;
+  if (cl == 1) {
+    // two CTAs per SM; with fewer tiles than that a tile is cut, and its finisher folds the pieces, four at a time: a
+    // stage at 0.7 us against 0.12 us per piece (fitted on 1024 x 28672: 74 / 148 / 296 CTAs 12.2 / 9.1 / 9.2 us)
+    grid = std::min(2 * nsm, p.total_iters);
+    if (p.n_tiles <= grid) grid = pick_workers(p.n_tiles, p.k_iters, grid, 0.7 * KS / 256, 0.12);
+    p.iters_per_cta = (p.total_iters + grid - 1) / grid;
+    grid = (p.total_iters + p.iters_per_cta - 1) / p.iters_per_cta;
+  }
+  if (pr.plan) {   // (in units of two CTAs, one SM's worth)
+    const int kernel = cl > 1 ? W4A16_KERNEL_DECODE_CLUSTER : KS == 256 ? W4A16_KERNEL_DECODE : W4A16_KERNEL_SINGLE;
+    *pr.plan = w4a16_plan_t{kernel, 16, KS, (grid + 1) / 2, cl > 1 ? cl / 2 : 2, 0, cl > 1 ? p.k_iters / (cl / 2) : 2 * p.iters_per_cta};
+    return W4A16_OK;
+  }
+  Maps mp;
+  if (!get_maps(pr, KS, Cfg::ROWS, GROUPED, false, mp, true)) return W4A16_ERR_CUDA;
+  if (!mp.a_box3d) return -2;
+  if (!get_scratch(pr, cl == 1 ? (size_t)grid * Cfg::ROWS * w4a16::TILE_N : 0, p)) return pr.fixed_partials ? W4A16_ERR_ARG : W4A16_ERR_CUDA;
+  attr[0].val.clusterDim.x = (unsigned)cl;
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.numAttrs = 2;
+  if (!cuda_ok(cudaLaunchKernelEx(&cfg, kern, mp.b, mp.a, mp.s, p, cl), "kernel launch (skinny)")) return W4A16_ERR_CUDA;
+  return W4A16_OK;
+}
+
+int launch_skinny_g(const Problem &pr) {
+  const bool g = pr.groupsize == 128;
+  if (pr.k % 256 == 0) return g ? launch_skinny<256, true>(pr) : launch_skinny<256, false>(pr);
+  return g ? launch_skinny<128, true>(pr) : launch_skinny<128, false>(pr);
 }
 
 // ---- large batches on CTA pairs (cta_group::2): see w4a16_kernel_2sm.cuh
@@ -717,6 +821,14 @@ int launch_decode_g(const Problem &pr) {
 int dispatch_tc(const Problem &pr) {
   // batch tile = UMMA N; the k per stage is as deep as the activation tile allows (fewer, larger TMAs)
   const bool k256 = (pr.k % 256) == 0, k128 = (pr.k % 128) == 0;
+  // Up to 8 rows: mma.sync on half-SM CTAs (us per launch in a chain at m = 1, before -> after: 512 x 1024 5.0 -> 2.2,
+  // 1024 x 8192 7.3 -> 4.3, 4096 x 4096 6.5 -> 4.8, 12288 x 4096 9.6 -> 7.6, 22016 x 4096 13.5 -> 10.5, 3328 x 4480 8.5 -> 4.5,
+  // 8192 x 28672 26.0 -> 22.4, 57344 x 8192 44.6 -> 39.8).  At 16 rows its MMAs double and the tcgen05 kernel wins (4096 x 4096
+  // 6.7 against 7.0, 22016 x 4096 13.5 against 16.8 us).
+  if (pr.m <= 8 && k128 && g_use_skinny && pr.sms <= 0 && pr.c_ld == 0 && !pr.orphan_finisher) {
+    const int rc = launch_skinny_g(pr);
+    if (rc != -2) return rc;
+  }
   if (pr.m <= 16 && k256 && g_use_decode) {   // the HBM-bound case has a kernel of its own
     // few tiles and no split count from the caller: one cluster per tile
     if (g_use_cluster && pr.sms <= 0 && pr.c_ld == 0 && !pr.orphan_finisher) {

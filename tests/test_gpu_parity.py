@@ -452,6 +452,23 @@ def test_device_quantize_pack_edges(n, k, groupsize):
     assert np.array_equal(sp_dev.cpu().numpy().view(np.uint16), sp_host.view(np.uint16))
 
 
+@pytest.mark.parametrize("n,k", [(128, 128), (256, 512), (128, 11008), (4096, 4096), (8192, 8192), (1280, 4480), (2304, 1152),
+                                 (37888, 256), (38144, 640), (1024, 28672)])
+@pytest.mark.parametrize("m,groupsize", [(1, 128), (5, -1), (8, 128)])
+def test_up_to_8_rows(m, n, k, groupsize):
+    """The kernel for up to 8 rows: one stage; clusters of 4 and 8, also with uneven shares; k an odd multiple of 128; a tile
+    cut many ways; as many tiles as CTAs and a few more; fewer rows than ranks of a cluster."""
+    if groupsize == 128 and k == 128:
+        groupsize = -1      # one group of 128 is the per-channel layout
+    A, q, s = orc.make_problem(m, n, k, groupsize, seed=n + k + m)
+    At, Bt, st = pack_problem(A, q, s)
+    C = run_mul(At, Bt, st, m, n)
+    assert torch.equal(C, run_mul(At, Bt, st, m, n))
+    cols = np.r_[0:128, n - 128:n] if n * k > 1 << 24 else np.arange(n)     # oracle on the first and last tile only
+    ref = orc.c_gemm(A, np.ascontiguousarray(q[:, cols]), np.ascontiguousarray(s[:, cols]), groupsize)
+    check(C[:, torch.from_numpy(cols).to(C.device)], ref, "m=%d n=%d k=%d g=%d" % (m, n, k, groupsize))
+
+
 def test_pair_kernel_dependent_chain_graph_replay():
     """Two large-batch GEMMs (CTA-pair kernel) where the first one's output is the second one's activations,
     eagerly and over CUDA-graph replays; the oracle is evaluated on column windows, fed with the device's own
