@@ -10,6 +10,7 @@
 
 #include <algorithm>
 #include <array>
+#include <atomic>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -97,6 +98,7 @@ struct StreamCtx {
 constexpr int MAX_GRID = 256;
 
 std::mutex g_mu;
+std::atomic<uint64_t> g_launches{0};   // GEMMs and peer barriers this process has begun to launch, on any stream
 std::map<std::pair<int, cudaStream_t>, StreamCtx> g_ctx;
 int g_sm_count[64] = {0};
 
@@ -165,6 +167,8 @@ struct Problem {
   // tile also goes to the same place of n_extra further buffers
   int c_ld = 0, c_col0 = 0, n_extra = 0;
   void *const *C_extra = nullptr;   // device table of the n_extra further buffers
+  // set only by the call with host buffers: the result goes there too (page-locked, as addressed from the device)
+  void *C2 = nullptr;
   // set only by w4a16_plan: describe the launch instead of making it (no CUDA call on that path)
   w4a16_plan_t *plan = nullptr;
   int plan_sms = 0;                 // SMs of the device the plan is for
@@ -177,6 +181,7 @@ int problem_sm_count(const Problem &pr) { return pr.plan ? pr.plan_sms : sm_coun
 
 void set_output(w4a16::Params &p, const Problem &pr) {
   p.C = static_cast<__half *>(pr.C);
+  p.C2 = static_cast<__half *>(pr.C2);
   p.c_ld = pr.c_ld > 0 ? pr.c_ld : pr.n;
   p.c_col0 = pr.c_col0;
   p.n_extra = pr.n_extra;
@@ -539,6 +544,7 @@ int launch_decode_cluster_o(const Problem &pr, int cl) {
   return -2;
 }
 int launch_decode_cluster_g(const Problem &pr, int cl) {
+  if (pr.C2) return launch_decode_cluster_o<w4a16::OUT_DUAL>(pr, cl);
   return use_tma_store(pr) ? launch_decode_cluster_o<w4a16::OUT_TMA>(pr, cl) : launch_decode_cluster_o<w4a16::OUT_PLAIN>(pr, cl);
 }
 
@@ -797,6 +803,7 @@ int launch_tc_g(const Problem &pr) {
   using namespace w4a16;
   const bool g = pr.groupsize == 128;
   if (pr.c_ld > 0) return g ? launch_tc<TM, KS, true, OUT_GATHER>(pr) : launch_tc<TM, KS, false, OUT_GATHER>(pr);
+  if (pr.C2) return g ? launch_tc<TM, KS, true, OUT_DUAL>(pr) : launch_tc<TM, KS, false, OUT_DUAL>(pr);
   if (use_tma_store(pr)) return g ? launch_tc<TM, KS, true, OUT_TMA>(pr) : launch_tc<TM, KS, false, OUT_TMA>(pr);
   return g ? launch_tc<TM, KS, true, OUT_PLAIN>(pr) : launch_tc<TM, KS, false, OUT_PLAIN>(pr);
 }
@@ -806,6 +813,7 @@ int launch_tc2_g(const Problem &pr) {
   using namespace w4a16;
   const bool g = pr.groupsize == 128;
   if (pr.c_ld > 0) return g ? launch_tc2<TM, KS, true, OUT_GATHER>(pr) : launch_tc2<TM, KS, false, OUT_GATHER>(pr);
+  if (pr.C2) return g ? launch_tc2<TM, KS, true, OUT_DUAL>(pr) : launch_tc2<TM, KS, false, OUT_DUAL>(pr);
   if (use_tma_store(pr)) return g ? launch_tc2<TM, KS, true, OUT_TMA>(pr) : launch_tc2<TM, KS, false, OUT_TMA>(pr);
   return g ? launch_tc2<TM, KS, true, OUT_PLAIN>(pr) : launch_tc2<TM, KS, false, OUT_PLAIN>(pr);
 }
@@ -814,11 +822,13 @@ int launch_decode_g(const Problem &pr) {
   using namespace w4a16;
   const bool g = pr.groupsize == 128;
   if (pr.c_ld > 0) return g ? launch_single<DecodeKernel<true, OUT_GATHER>>(pr) : launch_single<DecodeKernel<false, OUT_GATHER>>(pr);
+  if (pr.C2) return g ? launch_single<DecodeKernel<true, OUT_DUAL>>(pr) : launch_single<DecodeKernel<false, OUT_DUAL>>(pr);
   if (use_tma_store(pr)) return g ? launch_single<DecodeKernel<true, OUT_TMA>>(pr) : launch_single<DecodeKernel<false, OUT_TMA>>(pr);
   return g ? launch_single<DecodeKernel<true, OUT_PLAIN>>(pr) : launch_single<DecodeKernel<false, OUT_PLAIN>>(pr);
 }
 
 int dispatch_tc(const Problem &pr) {
+  if (!pr.plan) g_launches.fetch_add(1);
   // batch tile = UMMA N; the k per stage is as deep as the activation tile allows (fewer, larger TMAs)
   const bool k256 = (pr.k % 256) == 0, k128 = (pr.k % 128) == 0;
   // Up to 8 rows: mma.sync on half-SM CTAs (us per launch in a chain at m = 1, before -> after: 512 x 1024 5.0 -> 2.2,
@@ -986,7 +996,7 @@ bool device_is_current(int dev) {
 
 int gemm_entry(bool simt, const void *A, const void *B, void *C, const void *s, int prob_m, int prob_n, int prob_k,
                void *workspace, int groupsize, int dev, cudaStream_t stream, int thread_k, int thread_n, int sms,
-               int max_par) {
+               int max_par, void *C2 = nullptr) {
   (void)max_par;
   (void)workspace;  // the caller's lock array is not needed by this kernel and is left untouched (all zero)
   if (prob_m < 0 || prob_n < 0 || prob_k < 0) return W4A16_ERR_ARG;
@@ -1000,6 +1010,7 @@ int gemm_entry(bool simt, const void *A, const void *B, void *C, const void *s, 
   if (dev < 0 || dev >= 64) return W4A16_ERR_ARG;
   if (!device_is_current(dev)) return W4A16_ERR_ARG;
   Problem pr{A, B, s, C, prob_m, prob_n, prob_k, groupsize, dev, sms, stream};
+  pr.C2 = C2;
   return simt ? launch_simt(pr) : dispatch_tc(pr);
 }
 
@@ -1033,44 +1044,99 @@ extern "C" int w4a16_plan(int prob_m, int prob_n, int prob_k, int groupsize, int
 
 // The GEMM with HOST activations and HOST output: copy in, multiply, copy out, all enqueued on `stream`.
 //
-// Small host<->device copies through the copy engines cost about ten microseconds each on the stream (set-up and
-// completion, not bytes), which is more than a decode GEMM.  When both host buffers are page-locked (and therefore
-// addressable from the device) and the batch is small, the copies are done by the SMs instead:
-//   * a few CTAs read A_host over PCIe into A_stage; the kernel signals griddepcontrol.launch_dependents at once, so
-//     the GEMM behind it starts its prologue and weight prefetch meanwhile and waits for the copy (griddepcontrol.wait)
-//     only before it loads activations;
-//   * the GEMM's epilogue writes C rows straight into C_host (posted PCIe writes): no second copy, no C_stage.
-// That serves a caller who runs one layer after the other on ONE stream (measured: the four 7B layers at m = 16 in
-// 121 us instead of 162 us); with several streams the copy engines overlap one layer's copies with another layer's
-// kernel and the direct writes only lengthen the kernels (66 us against 59.5 us; copying only A with the SMs: 65 us), so it is opt-in:
-// W4A16_HOST_DIRECT=1 in the environment.
+// A host<->device copy through the copy engines costs its stream about ten microseconds whatever its size (set-up and
+// completion), twice per call: more than a decode GEMM.  So when both host buffers are page-locked (and therefore addressable
+// from the device) and small, the SMs do the copies:
+//   * a kernel of a few blocks reads A_host over PCIe into A_stage.  It lets the GEMM behind it start at once, which
+//     prefetches its weights meanwhile and waits for the copy only before it loads activations;
+//   * the GEMM's epilogue writes each result to C_stage and, over PCIe, to C_host.
+// The copy-in may run beside the previous calls' GEMMs when those are the last things this library has launched and neither
+// touches what the other writes; it ends only after the GEMM before it has, so whatever waits for a call has waited for
+// everything before it.  How many of the earlier calls may still be running then is bounded by nothing but the room on
+// the SMs, so their buffers are remembered since the last copy-in that waited first, eight calls at most.  (Any kernel of
+// other origin in between restores full stream order, unless it too lets its successor start early.)
+// Several streams side by side overlap one call's copy engines with another's kernel, and there the SMs are worth more than the
+// latency (four layers on four streams 50 us with copy engines, 66 us without): the SMs copy when the last call of this
+// kind, by whatever thread, was on the same stream.  Four 7B layers at m = 16 in order on one stream: 159 -> 77 us (87-93
+// with a copy-out kernel instead of the epilogue's second store, 105 when the copy-in always waits); at m = 1 99 -> 47 us.
 namespace {
-const bool g_host_direct = [] {
+// W4A16_HOST_DIRECT=0 in the environment always takes the copy engines, =1 never for page-locked buffers (A/B timing)
+const int g_host_direct = [] {
   const char *e = std::getenv("W4A16_HOST_DIRECT");
-  return e && e[0] == '1';
+  return (e && (e[0] == '0' || e[0] == '1')) ? e[0] - '0' : -1;
 }();
 
-__global__ void __launch_bounds__(512) copy_in_kernel(const uint4 *__restrict__ src, uint4 *__restrict__ dst, size_t n16) {
+// Larger copies than this go through the copy engines: their ten microseconds are little by then.
+constexpr size_t HOST_COPY_MAX = 4u << 20;
+constexpr int COPY_THREADS = 1024, COPY_FLY = 4;
+
+// 16 bytes per thread and load, COPY_FLY loads in flight
+__global__ void __launch_bounds__(COPY_THREADS) copy_in_kernel(const uint4 *__restrict__ src, uint4 *__restrict__ dst, size_t n16, int early) {
   sm100::pdl_launch_dependents();   // the GEMM behind this kernel orders itself with griddepcontrol.wait
-  const size_t stride = (size_t)gridDim.x * blockDim.x;
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n16; i += stride) dst[i] = src[i];
+  if (!early) sm100::pdl_wait_prior_grid();
+  const size_t stride = (size_t)gridDim.x * COPY_THREADS;
+  size_t i = (size_t)blockIdx.x * COPY_THREADS + threadIdx.x;
+  for (; i + (COPY_FLY - 1) * stride < n16; i += COPY_FLY * stride) {
+    uint4 v[COPY_FLY];
+#pragma unroll
+    for (int f = 0; f < COPY_FLY; ++f) v[f] = src[i + f * stride];
+#pragma unroll
+    for (int f = 0; f < COPY_FLY; ++f) dst[i + f * stride] = v[f];
+  }
+  for (; i < n16; i += stride) dst[i] = src[i];
+  sm100::pdl_wait_prior_grid();
 }
 
-// device address of a page-locked host buffer, or null when the buffer is pageable (looked up once per pointer)
-void *device_view_of_host(const void *host) {
-  static std::map<const void *, void *> cache;   // guarded by g_mu
-  std::lock_guard<std::mutex> lock(g_mu);
-  auto it = cache.find(host);
-  if (it != cache.end()) return it->second;
-  void *dptr = nullptr;
-  cudaPointerAttributes attr{};
-  if (cudaPointerGetAttributes(&attr, host) == cudaSuccess && attr.type == cudaMemoryTypeHost && attr.devicePointer)
-    dptr = attr.devicePointer;
-  else
+// Device address of a page-locked host buffer, or null.  Asked on every call: a buffer may have been freed and its
+// address come back as pageable memory.
+void *device_view_of_host(const void *host, size_t bytes) {
+  cudaPointerAttributes first{}, last{};
+  const char *h = static_cast<const char *>(host);
+  if (cudaPointerGetAttributes(&first, h) != cudaSuccess || cudaPointerGetAttributes(&last, h + bytes - 1) != cudaSuccess) {
     cudaGetLastError();   // a pageable pointer is not an error here
-  if (cache.size() >= 4096) cache.clear();
-  cache[host] = dptr;
-  return dptr;
+    return nullptr;
+  }
+  if (first.type != cudaMemoryTypeHost || last.type != cudaMemoryTypeHost || !first.devicePointer ||
+      static_cast<char *>(last.devicePointer) - static_cast<char *>(first.devicePointer) != (ptrdiff_t)(bytes - 1))
+    return nullptr;
+  return first.devicePointer;
+}
+
+bool overlap(const void *a, size_t na, const void *b, size_t nb) {
+  const uintptr_t x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b);
+  return x < y + nb && y < x + na;
+}
+
+// The last call with host buffers, and the buffers of all calls that may be unfinished when the next copy-in starts early:
+// those since the last copy-in that waited for everything before it (guarded by g_mu)
+struct HostBuffers {
+  const void *a_stage, *c_stage, *c_host;
+  size_t a_bytes, c_bytes;
+};
+struct HostChain {
+  bool any = false;
+  int dev = 0;
+  cudaStream_t stream = nullptr;
+  uint64_t launches = 0;                // g_launches after it, or 0 when its copies went through the copy engines
+  std::vector<HostBuffers> open;
+} g_host_chain;
+constexpr size_t HOST_CHAIN_MAX = 8;
+
+int launch_copy_in(const void *src, void *dst, size_t bytes, cudaStream_t st, int early) {
+  cudaLaunchConfig_t cfg = {};
+  // few SMs: one block per 64 KB, at most 16 (PCIe, not the SMs, bounds it), so that the GEMM's CTAs find theirs free
+  cfg.gridDim = dim3((unsigned)std::min<size_t>(16, (bytes + 65535) / 65536));
+  cfg.blockDim = dim3(COPY_THREADS);
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = g_use_pdl ? 1 : 0;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cuda_ok(cudaLaunchKernelEx(&cfg, copy_in_kernel, static_cast<const uint4 *>(src), static_cast<uint4 *>(dst), bytes / 16, early),
+                 "copy-in launch")
+             ? W4A16_OK
+             : W4A16_ERR_CUDA;
 }
 }  // namespace
 
@@ -1085,24 +1151,46 @@ extern "C" int w4a16_marlin_gemm_host(const void *A_host, const void *B, void *C
   if (chk != W4A16_OK) return chk;
   if (!A_host || !C_host || !A_stage || !C_stage) return W4A16_ERR_ARG;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const size_t a_bytes = sizeof(__half) * (size_t)prob_m * prob_k;
-  if (g_host_direct && prob_m <= 64 && (a_bytes & 15) == 0 && !(reinterpret_cast<uintptr_t>(A_stage) & 15)) {
-    void *dA = device_view_of_host(A_host), *dC = device_view_of_host(C_host);
-    if (dA && dC && !((reinterpret_cast<uintptr_t>(dA) | reinterpret_cast<uintptr_t>(dC)) & 15)) {
-      if (!device_is_current(dev)) return W4A16_ERR_ARG;
-      copy_in_kernel<<<4, 512, 0, st>>>(static_cast<const uint4 *>(dA), static_cast<uint4 *>(A_stage), a_bytes / 16);
-      if (!cuda_ok(cudaGetLastError(), "copy-in launch")) return W4A16_ERR_CUDA;
-      return gemm_entry(false, A_stage, B, dC, s, prob_m, prob_n, prob_k, workspace, groupsize, dev, st, -1, -1, sms, 16);
-    }
+  const size_t a_bytes = sizeof(__half) * (size_t)prob_m * prob_k, c_bytes = sizeof(__half) * (size_t)prob_m * prob_n;
+
+  bool direct = false;
+  int early = 0;
+  if (g_host_direct != 0 && a_bytes <= HOST_COPY_MAX && c_bytes <= HOST_COPY_MAX) {
+    std::lock_guard<std::mutex> lock(g_mu);
+    const HostChain &l = g_host_chain;
+    const bool same = l.any && l.dev == dev && l.stream == st;
+    direct = g_host_direct == 1 || same;
+    early = direct && same && l.launches != 0 && l.launches == g_launches.load() && l.open.size() < HOST_CHAIN_MAX;
+    for (const HostBuffers &o : l.open)   // what this call's copy-in reads and writes
+      if (overlap(A_host, a_bytes, o.c_host, o.c_bytes) || overlap(A_stage, a_bytes, o.c_stage, o.c_bytes) ||
+          overlap(A_stage, a_bytes, o.a_stage, o.a_bytes))
+        early = 0;
   }
-  if (!cuda_ok(cudaMemcpyAsync(A_stage, A_host, a_bytes, cudaMemcpyHostToDevice, st), "cudaMemcpyAsync(A)"))
-    return W4A16_ERR_CUDA;
-  const int rc = gemm_entry(false, A_stage, B, C_stage, s, prob_m, prob_n, prob_k, workspace, groupsize, dev, st, -1, -1,
-                            sms, 16);
+  void *dA = nullptr, *dC = nullptr;
+  if (direct) {
+    dA = device_view_of_host(A_host, a_bytes);
+    dC = dA ? device_view_of_host(C_host, c_bytes) : nullptr;
+    direct = dC && !((reinterpret_cast<uintptr_t>(dA) | reinterpret_cast<uintptr_t>(dC) | reinterpret_cast<uintptr_t>(A_stage)) & 15);
+    if (direct && !device_is_current(dev)) return W4A16_ERR_ARG;
+  }
+  int rc;
+  if (direct)
+    rc = launch_copy_in(dA, A_stage, a_bytes, st, early);
+  else
+    rc = cuda_ok(cudaMemcpyAsync(A_stage, A_host, a_bytes, cudaMemcpyHostToDevice, st), "cudaMemcpyAsync(A)") ? W4A16_OK : W4A16_ERR_CUDA;
   if (rc != W4A16_OK) return rc;
-  if (!cuda_ok(cudaMemcpyAsync(C_host, C_stage, sizeof(__half) * (size_t)prob_m * prob_n, cudaMemcpyDeviceToHost, st),
-               "cudaMemcpyAsync(C)"))
-    return W4A16_ERR_CUDA;
+  rc = gemm_entry(false, A_stage, B, C_stage, s, prob_m, prob_n, prob_k, workspace, groupsize, dev, st, -1, -1, sms, 16,
+                  direct ? dC : nullptr);
+  if (rc != W4A16_OK) return rc;
+  if (!direct && !cuda_ok(cudaMemcpyAsync(C_host, C_stage, c_bytes, cudaMemcpyDeviceToHost, st), "cudaMemcpyAsync(C)")) return W4A16_ERR_CUDA;
+  std::lock_guard<std::mutex> lock(g_mu);
+  HostChain &l = g_host_chain;
+  l.any = true;
+  l.dev = dev;
+  l.stream = st;
+  l.launches = direct ? g_launches.load() : 0;
+  if (!early) l.open.clear();
+  l.open.push_back(HostBuffers{A_stage, C_stage, C_host, a_bytes, c_bytes});
   return W4A16_OK;
 }
 
@@ -1420,6 +1508,7 @@ extern "C" int w4a16_peer_barrier(void *const *flags, int world, int rank, int d
   }
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   int *status = nullptr;
+  g_launches.fetch_add(1);
   {
     std::lock_guard<std::mutex> lock(g_mu);
     StreamCtx *ctx = get_ctx(dev, st, 0);

@@ -81,6 +81,7 @@ struct Params {
   int dp_waves, sk_tile0, workers, m_fast;
   const __half *s;                      // scales (read directly by the epilogue when per-channel)
   __half *C;
+  __half *C2;                           // OUT_DUAL only: where else the result goes, [m][n]
   uint32_t *partials;                   // [gridDim.x][TM][128] fp32 partial tiles; PARTIAL_IDLE between launches
   int *status;                          // 0, or STATUS_TIMEOUT | (site << 8)
   uint64_t wait_ns;                     // every device-side wait gives up after this long (WAIT_LIMIT_NS by default)
@@ -97,6 +98,15 @@ static_assert(sizeof(Params) <= 128, "the kernels take four tensor maps and this
 constexpr int OUT_PLAIN = 0;    // 2-byte global stores from registers, 64 contiguous bytes per warp and row
 constexpr int OUT_GATHER = 1;   // staged in shared memory, written by rows to C and to the other ranks' buffers
 constexpr int OUT_TMA = 2;      // staged in shared memory, one cp.async.bulk.tensor store per 16-row x 128-column chunk
+constexpr int OUT_DUAL = 3;     // as OUT_PLAIN, and the same to C2 (page-locked host memory); an instantiation of its own,
+                                // since a test per store, or a second pass over the tile, cost the decode kernel 2-4 %
+__host__ __device__ constexpr bool staged_output(int out) { return out == OUT_GATHER || out == OUT_TMA; }
+
+template <int OUT>
+__device__ __forceinline__ void store_c(const Params &p, size_t at, __half h) {
+  p.C[at] = h;
+  if constexpr (OUT == OUT_DUAL) p.C2[at] = h;
+}
 
 // Gathering epilogue, cooperative form used by the epilogue warps.  A warp owns 32 weight columns (its TMEM lane
 // quadrant), so on its own it can only write 64 contiguous bytes per output row, and peer stores of that size reach
@@ -197,7 +207,7 @@ struct Config {
   static constexpr int WBUFS = WBUFS_RAW > 8 ? 8 : WBUFS_RAW;  // TMEM operand ring depth
   static_assert(WBUFS >= 2, "TMEM budget");
   static constexpr int BAR_BYTES = 1024;
-  static constexpr int GATHER_BYTES = OUT != OUT_PLAIN ? GATHER_SLAB_BYTES : 0;   // output staging of the gathering / TMA-store epilogue
+  static constexpr int GATHER_BYTES = staged_output(OUT) ? GATHER_SLAB_BYTES : 0;   // output staging of the gathering / TMA-store epilogue
   static constexpr int SMEM_MAX = 227 * 1024;
   static constexpr int STAGES_RAW = (SMEM_MAX - BAR_BYTES - GATHER_BYTES - 1024) / STAGE_BYTES;
   static constexpr int STAGES = STAGES_RAW > 12 ? 12 : STAGES_RAW;
@@ -322,7 +332,7 @@ w4a16_tc_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant__
   constexpr int NDQ = Cfg::NDQ;
   // dequant warps help to finish a split tile (see the epilogue); not in the gathering form, whose four epilogue
   // warps write every chunk together
-  constexpr bool HELP = TM >= 64 && OUT == OUT_PLAIN;
+  constexpr bool HELP = TM >= 64 && !staged_output(OUT);
   constexpr int PRODUCER_WARP = NDQ + EPI_WARPS, MMA_WARP = NDQ + EPI_WARPS + 1;
   constexpr uint32_t STAGE_TX = Cfg::W_BYTES + Cfg::A_BYTES + (GROUPED ? Cfg::S_BYTES : 0);
 
@@ -545,7 +555,7 @@ w4a16_tc_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant__
             const int mm = m0 + c0 + i;
             __half h = __float2half(__uint_as_float(v[i]));
             if (!GROUPED) h = __hmul(h, sch);  // per-channel scale after the fp16 convert (marlin_cute_trait.h:764-769)
-            if (mm < p.m) p.C[(size_t)mm * p.n + n0 + row] = h;
+            if (mm < p.m) store_c<OUT>(p, (size_t)mm * p.n + n0 + row, h);
           }
         }
         if (!ok) give_up(p, abort, 9);
@@ -619,7 +629,7 @@ w4a16_tc_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant__
               const int mm = m0 + c0 + i;
               __half h = __float2half(__uint_as_float(v[i]));
               if (!GROUPED) h = __hmul(h, sch);  // per-channel scale after the fp16 convert (marlin_cute_trait.h:764-769)
-              if (mm < p.m) p.C[(size_t)mm * p.n + n0 + row] = h;
+              if (mm < p.m) store_c<OUT>(p, (size_t)mm * p.n + n0 + row, h);
             }
           }
         }

@@ -39,7 +39,7 @@ struct Config2 {
   static constexpr int WBUFS = WBUFS_RAW > 4 ? 4 : WBUFS_RAW;
   static_assert(WBUFS >= 2, "TMEM budget");
   static constexpr int BAR_BYTES = 1024;
-  static constexpr int GATHER_BYTES = OUT != OUT_PLAIN ? GATHER_SLAB_BYTES : 0;
+  static constexpr int GATHER_BYTES = staged_output(OUT) ? GATHER_SLAB_BYTES : 0;
   static constexpr int SMEM_MAX = 227 * 1024;
   static constexpr int STAGES_RAW = (SMEM_MAX - BAR_BYTES - GATHER_BYTES - 1024) / STAGE_BYTES;
   static constexpr int STAGES = STAGES_RAW > 8 ? 8 : STAGES_RAW;
@@ -122,7 +122,7 @@ w4a16_tc2_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant_
   using namespace sm100;
   constexpr int S = Cfg::STAGES, NDQ = Cfg::NDQ, KS = Cfg::KS;
   constexpr int PRODUCER_WARP = NDQ + EPI_WARPS, MMA_WARP = NDQ + EPI_WARPS + 1;
-  constexpr bool HELP = TM >= 64 && OUT == OUT_PLAIN;   // dequant warps help to finish a split tile (as in the single-CTA kernel)
+  constexpr bool HELP = TM >= 64 && !staged_output(OUT);   // dequant warps help to finish a split tile (as in the single-CTA kernel)
   constexpr uint32_t WS_TX = Cfg::W_BYTES + (GROUPED ? Cfg::S_BYTES : 0);
 
   extern __shared__ uint8_t smem_raw[];
@@ -287,7 +287,7 @@ w4a16_tc2_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant_
             const int mm = m0 + c0 + i;
             __half h = __float2half(__uint_as_float(v[i]));
             if (!GROUPED) h = __hmul(h, sch);  // per-channel scale after the fp16 convert (marlin_cute_trait.h:764-769)
-            if (mm < p.m) p.C[(size_t)mm * p.n + n0 + row] = h;
+            if (mm < p.m) store_c<OUT>(p, (size_t)mm * p.n + n0 + row, h);
           }
         }
         if (!ok) give_up(p, abort, 19);
@@ -352,7 +352,7 @@ w4a16_tc2_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant_
               const int mm = m0 + c0 + i;
               __half h = __float2half(__uint_as_float(v[i]));
               if (!GROUPED) h = __hmul(h, sch);  // per-channel scale after the fp16 convert (marlin_cute_trait.h:764-769)
-              if (mm < p.m) p.C[(size_t)mm * p.n + n0 + row] = h;
+              if (mm < p.m) store_c<OUT>(p, (size_t)mm * p.n + n0 + row, h);
             }
           }
         }

@@ -442,7 +442,7 @@ w4a16_decode_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_consta
             const int mm = m0 + i;
             __half hv = __float2half(__uint_as_float(v[i]));
             if (!GROUPED) hv = __hmul(hv, sch);  // per-channel scale after the fp16 convert (marlin_cute_trait.h:764-769)
-            if (mm < p.m) p.C[(size_t)mm * p.n + n0 + row] = hv;
+            if (mm < p.m) store_c<OUT>(p, (size_t)mm * p.n + n0 + row, hv);
           }
         }
       }

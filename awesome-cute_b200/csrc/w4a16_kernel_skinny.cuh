@@ -357,8 +357,10 @@ w4a16_skinny_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_consta
       lo = __hmul2(lo, __halves2half2(sc[0], sc[1]));
       hi = __hmul2(hi, __halves2half2(sc[2], sc[3]));
     }
-    *reinterpret_cast<uint2 *>(p.C + (size_t)row * p.n + n0 + 4 * lane) =
-        make_uint2(*reinterpret_cast<uint32_t *>(&lo), *reinterpret_cast<uint32_t *>(&hi));
+    const uint2 out = make_uint2(*reinterpret_cast<uint32_t *>(&lo), *reinterpret_cast<uint32_t *>(&hi));
+    const size_t at = (size_t)row * p.n + n0 + 4 * lane;
+    *reinterpret_cast<uint2 *>(p.C + at) = out;
+    if (p.C2) *reinterpret_cast<uint2 *>(p.C2 + at) = out;
   }
 }
 

@@ -100,11 +100,14 @@ int w4a16_marlin_gemm_builtin_scratch(const void *A, const void *B, void *C, con
  * resident, as the reference's Layer keeps them, gemm/marlin_gemm/marlin.py:82-85).  It is the host-tensor
  * form of the reference's  mul()  (gemm/marlin_gemm/marlin.py:11-24), which the reference only offers for
  * device tensors.  Returns like w4a16_marlin_gemm; the caller synchronises `stream` before reading C_host.
- * With W4A16_HOST_DIRECT=1 in the environment, page-locked host buffers and prob_m <= 64, the copies do not go through
- * the copy engines (about ten microseconds of stream time each, more than a decode GEMM): a small kernel reads A_host
- * over PCIe into A_stage while the GEMM behind it already prefetches its weights, and the GEMM writes its result rows
- * straight into C_host; C_stage is then not touched.  It pays on a single stream (layers run one after the other) and
- * costs where several streams already overlap copies with kernels, hence opt-in.
+ * With page-locked host buffers of at most 4 MB each, a call on the same stream as the last call of this kind does not go
+ * through the copy engines (about ten microseconds of stream time per copy, more than a decode GEMM): a small kernel
+ * reads A_host over PCIe into A_stage while the GEMM behind it already prefetches its weights, and the GEMM writes its
+ * result rows into C_stage and C_host.  Its copy-in may overlap the previous such calls' GEMMs on the stream where their
+ * buffers do not overlap; stream order holds for all work of other origin, except a kernel that uses
+ * griddepcontrol.launch_dependents before it has finished with A_host or A_stage.  Calls that alternate between streams
+ * keep the copy engines, which overlap one stream's copies with another's kernels.  W4A16_HOST_DIRECT=0 in the environment
+ * always takes the copy engines, =1 never.
  */
 int w4a16_marlin_gemm_host(const void *A_host, const void *B, void *C_host, const void *s, int prob_m, int prob_n,
                            int prob_k, void *workspace, int groupsize, int dev, void *stream, void *A_stage,

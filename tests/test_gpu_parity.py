@@ -452,6 +452,54 @@ def test_device_quantize_pack_edges(n, k, groupsize):
     assert np.array_equal(sp_dev.cpu().numpy().view(np.uint16), sp_host.view(np.uint16))
 
 
+@pytest.mark.parametrize("m", [1, 8, 13, 40, 96])
+@pytest.mark.parametrize("shared", [False, True])
+def test_host_calls_in_a_chain(m, shared):
+    """Calls with host buffers one after the other on one stream: each layer reads the host buffer that the one before has
+    written, with staging buffers of its own or shared, over several passes; then each layer from a buffer of its own.
+    Results are those of mul() bit for bit, in C_host and in the staging buffer."""
+    dims = [512, 1024, 256, 512]
+    rng = np.random.default_rng(m)
+    layers = []
+    for i in range(3):
+        A, q, s = orc.make_problem(1, dims[i + 1], dims[i], 128, seed=i)
+        _, Bt, st = pack_problem(A, q, s * np.float16(0.25))
+        layers.append((Bt, st, torch.zeros(dims[i + 1] // 128 * 16, dtype=torch.int, device=DEV)))
+    big = max(dims) * m
+    own = lambda n: torch.zeros((m, n), dtype=torch.half, device=DEV)
+    pool = [torch.zeros(big, dtype=torch.half, device=DEV) for _ in range(2)]
+    stage = [((pool[0][:m * dims[i]].view(m, dims[i]), pool[1][:m * dims[i + 1]].view(m, dims[i + 1])) if shared else
+              (own(dims[i]), own(dims[i + 1]))) for i in range(3)]
+    host = [torch.zeros((m, d), dtype=torch.half).pin_memory() for d in dims]
+    stream = torch.cuda.Stream()
+    ops = [pkg.HostGemm(host[i], B, host[i + 1], s, ws, *stage[i], stream=stream) for i, (B, s, ws) in enumerate(layers)]
+    for _ in range(12):
+        x = torch.from_numpy((rng.standard_normal((m, dims[0])) * 0.5).astype(np.float16))
+        host[0].copy_(x)
+        for op in ops:
+            op()
+        stream.synchronize()
+        want = x.to(DEV)
+        for i, (B, s, ws) in enumerate(layers):
+            nxt = torch.zeros((m, dims[i + 1]), dtype=torch.half, device=DEV)
+            pkg.mul(want, B, nxt, s, ws)
+            want = nxt
+            assert torch.equal(want.cpu(), host[i + 1])
+        assert torch.equal(want, stage[2][1])
+    ins = [torch.from_numpy(rng.standard_normal((m, dims[i])).astype(np.float16)).pin_memory() for i in range(3)]
+    outs = [torch.zeros((m, dims[i + 1]), dtype=torch.half).pin_memory() for i in range(3)]
+    ops = [pkg.HostGemm(ins[i], B, outs[i], s, ws, *stage[i], stream=stream) for i, (B, s, ws) in enumerate(layers)]
+    for _ in range(20):
+        for op in ops:
+            op()
+    stream.synchronize()
+    for i, (B, s, ws) in enumerate(layers):
+        C = torch.zeros((m, dims[i + 1]), dtype=torch.half, device=DEV)
+        pkg.mul(ins[i].to(DEV), B, C, s, ws)
+        assert torch.equal(C.cpu(), outs[i])
+    pkg.device_status(0)
+
+
 @pytest.mark.parametrize("n,k", [(128, 128), (256, 512), (128, 11008), (4096, 4096), (8192, 8192), (1280, 4480), (2304, 1152),
                                  (37888, 256), (38144, 640), (1024, 28672)])
 @pytest.mark.parametrize("m,groupsize", [(1, 128), (5, -1), (8, 128)])
