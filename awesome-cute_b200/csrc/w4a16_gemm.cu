@@ -521,7 +521,7 @@ int launch_decode_cluster(const Problem &pr) {
 
 // W4A16_TMA_STORE=0 / 1 in the environment picks how finished tiles of the plain GEMM reach C: 2-byte stores from
 // registers, or staged in shared memory and stored by the copy engine (cp.async.bulk.tensor).  Both are compiled
-// and tested; the default is the one measured faster (see tma_store_default).  The kernel for up to 8 rows has one form: a warp
+// and tested; the default is the one measured faster (see tma_store_default).  The mma.sync kernel has one form: a warp
 // stores 256 contiguous bytes.
 const int g_tma_store = [] {
   const char *e = std::getenv("W4A16_TMA_STORE");
@@ -548,18 +548,43 @@ int launch_decode_cluster_g(const Problem &pr, int cl) {
   return use_tma_store(pr) ? launch_decode_cluster_o<w4a16::OUT_TMA>(pr, cl) : launch_decode_cluster_o<w4a16::OUT_PLAIN>(pr, cl);
 }
 
-// ---- up to 8 rows on CTAs of half an SM: see w4a16_kernel_skinny.cuh
+// ---- up to 8 rows, and some of up to 16, on CTAs of half an SM: see w4a16_kernel_skinny.cuh
 // W4A16_SKINNY=0 in the environment keeps these batches on the other kernels (debugging aid, A/B timing)
 const bool g_use_skinny = [] {
   const char *e = std::getenv("W4A16_SKINNY");
   return !(e && e[0] == '0');
 }();
 
+// Cluster size of that kernel, 1 for its stream-K form, 0 where another kernel is better.  fit[c]: clusters of c CTAs that can
+// be resident together (null: as many as the SMs have room for).
+// Up to 8 rows: as large as fits two CTAs to an SM, while a rank keeps at most 12 stages of 256 k; deeper, the latency that
+// a cluster saves is less than what idle SMs cost (m = 1, us: 4096 x 4096 4.8 on clusters of 8, 5.2 on stream-K; 8192 x 8192
+// 8.8 / 9.3; 1024 x 8192 4.3 / 5.4; 8192 x 28672, 28 stages a rank, 23.2 / 22.4; 1024 x 28672, 14 stages a rank, 9.9 / 9.1).
+// 9 to 16 rows: twice the MMAs, so a rank takes less, and least where two share an SM; k an odd multiple of 128 has no
+// tcgen05 kernel of its own and stays here when there are enough tiles (m = 16, us, general kernel -> this one:
+// 12288 x 4224 16.4 -> 11.9, 8192 x 4224 11.5 -> 11.0; but 4096 x 4224 8.8 -> 10.3 on stream-K).
+int skinny_cluster(int mt, int n_tiles, int k, int ks, int nsm, const int *fit) {
+  const int k_iters = k / ks;
+  auto serves = [&](int c, int ctas, int most_k) {
+    return g_use_cluster && n_tiles * c <= ctas && k_iters >= c && k <= most_k * c && (!fit || fit[c] >= n_tiles);
+  };
+  if (mt == 1) {
+    for (int c = 8; c >= 4; c /= 2)
+      if (serves(c, 2 * nsm, 12 * 256)) return c;
+    return 1;
+  }
+  for (int c = 8; c >= 4; c /= 2)
+    if (serves(c, nsm, (c == 8 ? 12 : 6) * 128)) return c;
+  for (int c = 8; c >= 4; c /= 2)
+    if (serves(c, 2 * nsm, 4 * 128)) return c;
+  return k % 256 != 0 && n_tiles >= 64 ? 1 : 0;
+}
+
 // Returns -2 when the kernel does not serve the call.
-template <int KS, bool GROUPED>
+template <int MT, int KS, bool GROUPED>
 int launch_skinny(const Problem &pr) {
-  using Cfg = w4a16::SkinnyConfig<KS>;
-  auto kern = w4a16::w4a16_skinny_kernel<KS, GROUPED>;
+  using Cfg = w4a16::SkinnyConfig<MT, KS>;
+  auto kern = w4a16::w4a16_skinny_kernel<MT, KS, GROUPED>;
   static bool attr_done[64] = {false};
   static int fit[64][9];                 // clusters of 4, 8 CTAs that can be resident together
   const int nsm = problem_sm_count(pr);
@@ -603,14 +628,8 @@ int launch_skinny(const Problem &pr) {
   set_output(p, pr);
   p.wait_ns = pr.wait_ns;
 
-  // Few tiles: one cluster per tile, as large as fits (two CTAs per SM), while a rank keeps at most 12 stages of 256 k;
-  // deeper, the latency that a cluster saves is less than what idle SMs cost (m = 1, us: 4096 x 4096 4.8 on clusters of 8,
-  // 5.2 on stream-K; 8192 x 8192 8.8 / 9.3; 1024 x 8192 4.3 / 5.4; 8192 x 28672, 28 stages a rank, 23.2 / 22.4;
-  // 1024 x 28672, 14 stages a rank, 9.9 / 9.1).
-  int cl = 1;
-  if (g_use_cluster)
-    for (int c = 4; c <= 8; c *= 2)
-      if (p.n_tiles * c <= 2 * nsm && p.k_iters >= c && p.k_iters * KS <= 12 * 256 * c && (pr.plan || fit[pr.dev][c] >= p.n_tiles)) cl = c;
+  const int cl = skinny_cluster(MT, p.n_tiles, pr.k, KS, nsm, pr.plan ? nullptr : fit[pr.dev]);
+  if (cl == 0) return -2;
   int grid = p.n_tiles * cl;
   if (cl == 1) {
     // two CTAs per SM; with fewer tiles than that a tile is cut, and its finisher folds the pieces, four at a time: a
@@ -621,7 +640,7 @@ int launch_skinny(const Problem &pr) {
     grid = (p.total_iters + p.iters_per_cta - 1) / p.iters_per_cta;
   }
   if (pr.plan) {   // (in units of two CTAs, one SM's worth)
-    const int kernel = cl > 1 ? W4A16_KERNEL_DECODE_CLUSTER : KS == 256 ? W4A16_KERNEL_DECODE : W4A16_KERNEL_SINGLE;
+    const int kernel = cl > 1 ? W4A16_KERNEL_DECODE_CLUSTER : pr.k % 256 == 0 ? W4A16_KERNEL_DECODE : W4A16_KERNEL_SINGLE;
     *pr.plan = w4a16_plan_t{kernel, 16, KS, (grid + 1) / 2, cl > 1 ? cl / 2 : 2, 0, cl > 1 ? p.k_iters / (cl / 2) : 2 * p.iters_per_cta};
     return W4A16_OK;
   }
@@ -638,8 +657,9 @@ int launch_skinny(const Problem &pr) {
 
 int launch_skinny_g(const Problem &pr) {
   const bool g = pr.groupsize == 128;
-  if (pr.k % 256 == 0) return g ? launch_skinny<256, true>(pr) : launch_skinny<256, false>(pr);
-  return g ? launch_skinny<128, true>(pr) : launch_skinny<128, false>(pr);
+  if (pr.m > 8) return g ? launch_skinny<2, 128, true>(pr) : launch_skinny<2, 128, false>(pr);
+  if (pr.k % 256 == 0) return g ? launch_skinny<1, 256, true>(pr) : launch_skinny<1, 256, false>(pr);
+  return g ? launch_skinny<1, 128, true>(pr) : launch_skinny<1, 128, false>(pr);
 }
 
 // ---- large batches on CTA pairs (cta_group::2): see w4a16_kernel_2sm.cuh
@@ -834,8 +854,11 @@ int dispatch_tc(const Problem &pr) {
   // Up to 8 rows: mma.sync on half-SM CTAs (us per launch in a chain at m = 1, before -> after: 512 x 1024 5.0 -> 2.2,
   // 1024 x 8192 7.3 -> 4.3, 4096 x 4096 6.5 -> 4.8, 12288 x 4096 9.6 -> 7.6, 22016 x 4096 13.5 -> 10.5, 3328 x 4480 8.5 -> 4.5,
   // 8192 x 28672 26.0 -> 22.4, 57344 x 8192 44.6 -> 39.8).  At 16 rows its MMAs double and the tcgen05 kernel wins (4096 x 4096
-  // 6.7 against 7.0, 22016 x 4096 13.5 against 16.8 us).
-  if (pr.m <= 8 && k128 && g_use_skinny && pr.sms <= 0 && pr.c_ld == 0 && !pr.orphan_finisher) {
+  // 6.7 against 7.8, 22016 x 4096 13.5 against 16.9 us).
+  // 9 to 16 rows: where latency counts, and for k an odd multiple of 128 (m = 16, us: 512 x 2048 5.7 -> 4.1, 512 x 8192
+  // 9.1 -> 5.6, 4096 x 1024 5.6 -> 4.5, 1024 x 4480 8.6 -> 5.2; from 8 million weights on the kernels are level).
+  const bool few_weights = pr.k <= 8192 && ((long)pr.n * pr.k <= 7000000 || pr.n <= 12 * w4a16::TILE_N);
+  if (pr.m <= (!k256 || few_weights ? 16 : 8) && k128 && g_use_skinny && pr.sms <= 0 && !pr.orphan_finisher) {
     const int rc = launch_skinny_g(pr);
     if (rc != -2) return rc;
   }

@@ -81,7 +81,7 @@ struct Params {
   int dp_waves, sk_tile0, workers, m_fast;
   const __half *s;                      // scales (read directly by the epilogue when per-channel)
   __half *C;
-  __half *C2;                           // OUT_DUAL only: where else the result goes, [m][n]
+  __half *C2;                           // null, or (OUT_DUAL, and the mma.sync kernel) where else the result goes, [m][n]
   uint32_t *partials;                   // [gridDim.x][TM][128] fp32 partial tiles; PARTIAL_IDLE between launches
   int *status;                          // 0, or STATUS_TIMEOUT | (site << 8)
   uint64_t wait_ns;                     // every device-side wait gives up after this long (WAIT_LIMIT_NS by default)

@@ -172,8 +172,9 @@ int w4a16_device_status(int dev, void *stream);
 #define W4A16_KERNEL_PAIRS 2          /* one CTA pair per worker (256 weight columns per tile) */
 #define W4A16_KERNEL_DECODE 3         /* prob_m <= 16: one CTA per worker, stream-K or one whole tile each */
 #define W4A16_KERNEL_DECODE_CLUSTER 4 /* prob_m <= 16: one cluster per 128-column tile */
-/* prob_m <= 8 without an explicit `sms`: the CTAs take half an SM, and a pair of them counts as one below (a worker is two
- * CTAs; `workers` of the cluster form and the cluster size count pairs).  tile_rows is 16 there too: the tile's room is 8. */
+/* prob_m <= 8 without an explicit `sms`, and some problems of up to 16 rows, run on CTAs that take half an SM; a pair of
+ * them counts as one below (a worker is two CTAs; `workers` of the cluster form and the cluster size count pairs).
+ * tile_rows is 16 there too: at prob_m <= 8 the tile's room is 8. */
 typedef struct {
   int kernel;            /* W4A16_KERNEL_* */
   int tile_rows;         /* batch rows per tile */

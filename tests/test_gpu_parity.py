@@ -501,10 +501,10 @@ def test_host_calls_in_a_chain(m, shared):
 
 
 @pytest.mark.parametrize("n,k", [(128, 128), (256, 512), (128, 11008), (4096, 4096), (8192, 8192), (1280, 4480), (2304, 1152),
-                                 (37888, 256), (38144, 640), (1024, 28672)])
-@pytest.mark.parametrize("m,groupsize", [(1, 128), (5, -1), (8, 128)])
-def test_up_to_8_rows(m, n, k, groupsize):
-    """The kernel for up to 8 rows: one stage; clusters of 4 and 8, also with uneven shares; k an odd multiple of 128; a tile
+                                 (37888, 256), (38144, 640), (1024, 28672), (8192, 512), (8192, 896)])
+@pytest.mark.parametrize("m,groupsize", [(1, 128), (5, -1), (8, 128), (9, -1), (16, 128)])
+def test_up_to_16_rows(m, n, k, groupsize):
+    """The half-SM kernel: one stage; clusters of 4 and 8, also with uneven shares; k an odd multiple of 128; a tile
     cut many ways; as many tiles as CTAs and a few more; fewer rows than ranks of a cluster."""
     if groupsize == 128 and k == 128:
         groupsize = -1      # one group of 128 is the per-channel layout
