@@ -73,7 +73,8 @@ struct DecodeConfig {
 };
 
 struct DecodeBars {  // lives in shared memory
-  uint64_t full[12];
+  uint64_t full[12];     // weights and scales of a stage landed
+  uint64_t afull[12];    // its activations landed
   uint64_t empty[12];
   uint64_t wfull[4];
   uint64_t wempty[4];
@@ -100,7 +101,7 @@ w4a16_decode_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_consta
   using namespace sm100;
   constexpr int S = Cfg::STAGES, NDQ = Cfg::NDQ, TM = Cfg::TM, KS = Cfg::KS;
   constexpr int PRODUCER_WARP = NDQ + EPI_WARPS, MMA_WARP = NDQ + EPI_WARPS + 1;   // first of NMMA issuer warps
-  constexpr uint32_t STAGE_TX = Cfg::W_BYTES + Cfg::A_BYTES + (GROUPED ? Cfg::S_BYTES : 0);
+  constexpr uint32_t WS_TX = Cfg::W_BYTES + (GROUPED ? Cfg::S_BYTES : 0);
   constexpr int PRE = 3;           // stages requested before the CTA-wide sync of the prologue (one per dequant set)
 
   extern __shared__ uint8_t smem_raw[];
@@ -132,12 +133,13 @@ w4a16_decode_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_consta
 
   auto issue_weights = [&](int st, int n_idx, int kk) {   // packed weights + group scales: immutable parameters
     const uint32_t full = smem_u32(&bars->full[st]);
-    mbar_expect_tx(full, STAGE_TX);
+    mbar_expect_tx(full, WS_TX);
     tma_load_3d(smem_u32(sW) + st * Cfg::W_BYTES, &tmB, 0, n_idx * 8, kk * (KS / 16), full);
     if (GROUPED) tma_load_2d(smem_u32(sS) + st * Cfg::S_BYTES, &tmS, n_idx * TILE_N, kk * Cfg::GROUPS, full);
   };
   auto issue_acts = [&](int st, int m0, int kk) {         // activations: may be the previous kernel's output
-    const uint32_t full = smem_u32(&bars->full[st]);
+    const uint32_t full = smem_u32(&bars->afull[st]);
+    mbar_expect_tx(full, Cfg::A_BYTES);
     if (p.a_box3d) {
       tma_load_3d(smem_u32(sA) + st * Cfg::A_BYTES, &tmA, 0, m0, kk * Cfg::KCHUNKS, full);
     } else {
@@ -155,6 +157,7 @@ w4a16_decode_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_consta
     // one barrier (or two) per lane, so that the first TMA can go out a few hundred clocks earlier
     if (lane < S) {
       mbar_init(smem_u32(&bars->full[lane]), 1);
+      mbar_init(smem_u32(&bars->afull[lane]), 1);
       // a stage is free when its dequant set has converted it, the MMAs that read its activations have completed
       // and (group scales) the epilogue warps have taken its scales
       mbar_init(smem_u32(&bars->empty[lane]), 4 + 1 + (GROUPED ? EPI_WARPS : 0));
@@ -180,7 +183,6 @@ w4a16_decode_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_consta
     pro_kk = it_begin - pro_tile * p.k_iters;
     pro_nidx = pro_tile % p.n_tiles;
     pro_m0 = (pro_tile / p.n_tiles) * TM;
-    bar_arrive(1, 64);             // barriers exist: the MMA warp may issue the activation loads (it waits, we do not)
     // Only the first PRE stages before the CTA-wide sync: issuing a TMA costs ~100 clocks, a whole ring-full would
     // hold the dequant warps at the sync for a microsecond, past the time the first stage lands.
     const int pre = min(PRE, nsteps);
@@ -197,19 +199,6 @@ w4a16_decode_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_consta
     if (lane == 0) { tma_prefetch_desc(&tmA); }
     tmem_alloc(smem_u32(&bars->tmem_base), Cfg::TMEM_COLS);
     tmem_relinquish();
-    bar_sync(1, 64);
-    pdl_wait_prior_grid();
-    int tile = it_begin / p.k_iters, kk = it_begin - tile * p.k_iters;
-    int m0 = (tile / p.n_tiles) * TM, nidx = tile % p.n_tiles;
-    const int pre = min(PRE, nsteps);
-    for (int i = 0; i < pre; ++i) {   // the activations of the stages whose weights the producer has requested
-      if (elect_one()) issue_acts(i, m0, kk);
-      __syncwarp();
-      if (++kk == p.k_iters) {
-        kk = 0;
-        if (++nidx == p.n_tiles) { nidx = 0; m0 += TM; }
-      }
-    }
   }
   tc_fence_before();
   __syncthreads();
@@ -507,11 +496,29 @@ w4a16_decode_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_consta
       for (int i = 0; i < issued; ++i) {
         const int sidx = pro_step - 1 - i;
         mbar_wait(smem_u32(&bars->full[sidx % S]), (sidx / S) & 1, &never, 200000000ull);
+        mbar_wait(smem_u32(&bars->afull[sidx % S]), (sidx / S) & 1, &never, 200000000ull);
       }
     }
   } else {
     // =========================================================== MMA issuer
     // Per stage: two groups of 8 MMAs (K = 16 each), each group into a fresh accumulator of the ring.
+    if (warp == MMA_WARP) {
+      // The activations of the stages whose weights the producer requested first, once the previous kernel of the stream has
+      // completed.  (Behind the CTA-wide sync and on barriers of their own: meanwhile the dequant warps fill the operand
+      // buffers.)
+      pdl_wait_prior_grid();
+      int tile = it_begin / p.k_iters, kk = it_begin - tile * p.k_iters;
+      int m0 = (tile / p.n_tiles) * TM, nidx = tile % p.n_tiles;
+      const int pre = min(PRE, nsteps);
+      for (int i = 0; i < pre; ++i) {   // the activations of the stages whose weights the producer has requested
+        if (elect_one()) issue_acts(i, m0, kk);
+        __syncwarp();
+        if (++kk == p.k_iters) {
+          kk = 0;
+          if (++nidx == p.n_tiles) { nidx = 0; m0 += TM; }
+        }
+      }
+    }
     constexpr uint32_t idesc = make_idesc_f16_f32(TILE_N, TM);
     bool ok = true;
     long long m_full = 0, m_wfull = 0, m_issue = 0, m_acc = 0;
@@ -519,8 +526,7 @@ w4a16_decode_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_consta
     for (int step = warp - MMA_WARP; step < nsteps && ok; step += Cfg::NMMA) {
       const int st = step % S, wb = step % Cfg::WBUFS, a = step % Cfg::NACC;
       const long long c1 = W4A16_CLK();
-      // The operand buffer is complete.  Its dequant warps waited for full[st] before they read the stage, so the
-      // activations of the stage have landed too (the barrier counts weights, scales and activations together).
+      if (!warp_wait(smem_u32(&bars->afull[st]), (step / S) & 1, abort, p.wait_ns)) { give_up(p, abort, 7); ok = false; break; }
       if (!warp_wait(smem_u32(&bars->wfull[wb]), (step / Cfg::WBUFS) & 1, abort, p.wait_ns)) { give_up(p, abort, 8); ok = false; break; }
       const long long c2 = W4A16_CLK();
       m_wfull += c2 - c1;
