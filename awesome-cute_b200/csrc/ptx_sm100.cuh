@@ -277,6 +277,16 @@ __device__ __forceinline__ uint32_t ld_shared_relaxed_cluster(uint32_t cta_addr)
   asm volatile("ld.relaxed.cluster.shared::cta.u32 %0, [%1];" : "=r"(v) : "r"(cta_addr) : "memory");
   return v;
 }
+// 4 or 16 bytes into another CTA's shared memory, counted there on `bar`: data and signal in one, no fence on either side
+__device__ __forceinline__ void st_async_f32(uint32_t cluster_addr, float v, uint32_t cluster_bar) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.f32 [%0], %1, [%2];" ::"r"(cluster_addr), "f"(v), "r"(cluster_bar)
+               : "memory");
+}
+__device__ __forceinline__ void st_async_f4(uint32_t cluster_addr, float4 v, uint32_t cluster_bar) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(cluster_addr),
+               "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w), "r"(cluster_bar)
+               : "memory");
+}
 // The two halves of the cluster barrier: a thread that has arrived may do other work before it waits.
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
 // (relaxed: for when what the other CTAs need to see was already released, e.g. barrier initialisation by
@@ -310,8 +320,8 @@ __device__ __forceinline__ void tc_mma_ts_pair(uint32_t d_tmem, uint32_t a_tmem,
       : "memory");
 }
 // arrive on the barrier at this shared-memory offset in BOTH CTAs of the pair once the pair's MMAs have completed
-__device__ __forceinline__ void tc_commit_pair(uint32_t bar) {
-  const uint16_t both = 3;
+// (`both`: the two CTAs' bits, by their ranks in the cluster)
+__device__ __forceinline__ void tc_commit_pair(uint32_t bar, uint16_t both) {
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
                ::"r"(bar), "h"(both)
                : "memory");

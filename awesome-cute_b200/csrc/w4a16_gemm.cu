@@ -521,8 +521,8 @@ int launch_decode_cluster(const Problem &pr) {
 
 // W4A16_TMA_STORE=0 / 1 in the environment picks how finished tiles of the plain GEMM reach C: 2-byte stores from
 // registers, or staged in shared memory and stored by the copy engine (cp.async.bulk.tensor).  Both are compiled
-// and tested; the default is the one measured faster (see tma_store_default).  The mma.sync kernel has one form: a warp
-// stores 256 contiguous bytes.
+// and tested; the default is the one measured faster (see tma_store_default).  The mma.sync kernel and
+// the clusters of CTA pairs have one form each.
 const int g_tma_store = [] {
   const char *e = std::getenv("W4A16_TMA_STORE");
   return (e && (e[0] == '0' || e[0] == '1')) ? e[0] - '0' : -1;
@@ -692,6 +692,120 @@ int pick_tile_order(int dev, double act_bytes, double weight_bytes, int n_tiles,
   return m_first < 0.9 * n_first ? 1 : 0;
 }
 
+// Few tiles, each cut into 2 to 4 pieces: one cluster of that many pairs per tile (the pieces exchange their partial sums over
+// distributed shared memory).  Returns -2 when such clusters cannot all be resident at once.
+template <int TM, int KS, bool GROUPED, int P>
+int launch_tc2_cluster(const Problem &pr) {
+  using Cfg = w4a16::Config2<TM, KS, w4a16::OUT_PLAIN, P>;
+  auto kern = w4a16::w4a16_tc2_kernel<TM, KS, GROUPED, w4a16::OUT_PLAIN, P>;
+  constexpr int smem = Cfg::SMEM_BYTES > 116 * 1024 ? Cfg::SMEM_BYTES : 116 * 1024;
+  static bool attr_done[64] = {false};
+  static int max_clusters[64] = {0};
+  const int nsm = problem_sm_count(pr);
+  if (nsm <= 0) return W4A16_ERR_CUDA;
+
+  w4a16::Params p{};
+  p.m = pr.m, p.n = pr.n, p.k = pr.k;
+  p.n_tiles = pr.n / (2 * w4a16::TILE_N);
+  p.m_tiles = (pr.m + TM - 1) / TM;
+  p.k_iters = pr.k / Cfg::KS;
+  const int tiles = p.n_tiles * p.m_tiles;
+  p.total_iters = tiles * p.k_iters;
+  p.iters_per_cta = (p.k_iters + P - 1) / P;   // per PAIR
+  p.workers = tiles * P;
+  p.s = static_cast<const __half *>(pr.s);
+  set_output(p, pr);
+  p.wait_ns = pr.wait_ns;
+  p.a_box3d = 1;
+  if (p.iters_per_cta * (P - 1) >= p.k_iters) return -2;   // (a pair without a stage)
+  if (pr.plan) {
+    if (2 * P * tiles > nsm) return -2;
+    *pr.plan = w4a16_plan_t{W4A16_KERNEL_PAIRS, TM, Cfg::KS, p.workers, 2, 0, p.iters_per_cta};
+    return W4A16_OK;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(2 * P * tiles));
+  cfg.blockDim = dim3((unsigned)Cfg::THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = pr.stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2 * P;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = g_use_pdl ? 1 : 0;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  {
+    std::lock_guard<std::mutex> lock(g_mu);
+    if (!attr_done[pr.dev]) {
+      if (!cuda_ok(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem), "cudaFuncSetAttribute"))
+        return W4A16_ERR_CUDA;
+      cudaLaunchConfig_t probe = cfg;
+      probe.gridDim = dim3((unsigned)(nsm / (2 * P) * (2 * P)));
+      int clusters = 0;
+      if (!cuda_ok(cudaOccupancyMaxActiveClusters(&clusters, kern, &probe), "cudaOccupancyMaxActiveClusters")) return W4A16_ERR_CUDA;
+      max_clusters[pr.dev] = clusters;
+      attr_done[pr.dev] = true;
+    }
+  }
+  if (max_clusters[pr.dev] < tiles) return -2;
+  Maps mp;
+  if (!get_maps(pr, Cfg::KS, Cfg::HALF_ROWS, GROUPED, false, mp)) return W4A16_ERR_CUDA;
+  if (!mp.a_box3d) return -2;
+  if (!get_scratch(pr, 0, p)) return W4A16_ERR_CUDA;   // the status word only
+  if (!cuda_ok(cudaLaunchKernelEx(&cfg, kern, mp.b, mp.a, mp.s, mp.c, p), "kernel launch (clusters of CTA pairs)")) return W4A16_ERR_CUDA;
+  return W4A16_OK;
+}
+
+// W4A16_PAIR_CLUSTER=0 in the environment keeps these problems on the stream-K form (A/B timing)
+const bool g_use_pair_cluster = [] {
+  const char *e = std::getenv("W4A16_PAIR_CLUSTER");
+  return !(e && e[0] == '0');
+}();
+
+// How many pairs work on a tile when there are fewer tiles than pairs, cheapest first, and 0 for the stream-K form with the
+// worker count of pick_workers.  Priced like that (a stage 0.45 us); what a cluster costs beside its stages hardly depends
+// on the tile, 0.3 us per further pair up to 64 rows and 0.7 us above, until clusters of six and eight CTAs take more than about
+// 90 SMs: they then wait for the previous launch to leave enough SMs of one GPC (1.5 us at 32 rows, 2.5 at 64, 2 above).  The
+// stream-K form pays its partial tiles and 3 us (1.5 above 64 rows, where every piece is priced at 2.2).  Above 64 rows a pair
+// keeps at least 12 stages unless pick_workers cuts shorter.  The limits on the SMs are what fits on 148 (clusters of 4 / 6 / 8:
+// 37 / 20 / 12 or more).  Measured, us, stream-K -> clusters: m = 24: 4096 x 4096 9.4 -> 7.2 (P = 2), 2048 x 8192 10.7 -> 8.6 (4),
+// 1024 x 2048 6.5 -> 4.2 (4); m = 48: 1024 x 8192 9.5 -> 7.5 (4); m = 77: 5120 x 5504 14.7 -> 12.0 (3); m = 128: 4096 x 4096
+// 13.7 -> 11.2 (2), 4096 x 11008 21.4 -> 18.5 (3); m = 512: 1024 x 28672 38.5 -> 35.1 (4).
+std::array<int, 3> pick_pair_clusters(int tm, int tiles, int k_iters, int pairs, int nsm) {
+  const double t_fix = tm >= 128 ? 2.2 : 0.5;
+  const int workers = pick_workers(tiles, k_iters, pairs, 0.45, t_fix);
+  const int per = (int)(((long)tiles * k_iters + workers - 1) / workers), pieces = (k_iters + per - 1) / per;
+  const bool lined_up = k_iters % per == 0 || tiles == 1;
+  const double stream_k = pieces == 1 ? 0.45 * per : 0.45 * per + (pieces - 1 + (lined_up ? 0 : 1)) * (tm >= 128 ? t_fix : 0.3) + (tm >= 128 ? 1.5 : 3.0);
+  std::array<std::pair<double, int>, 3> c;
+  for (int P = 2; P <= 4; ++P) {
+    const int ctas = 2 * P * tiles, share = (k_iters + P - 1) / P;
+    const bool fits = 100 * ctas <= (P == 2 ? 100 : P == 3 ? 82 : 66) * nsm && share * (P - 1) < k_iters;
+    double cost = 0.45 * share + (P - 2) * (tm >= 128 ? 0.7 : 0.3);
+    if (P > 2 && 100 * ctas > 60 * nsm) cost += tm >= 128 ? 2.0 : tm == 64 ? 2.5 : 1.5;
+    if (!fits || cost >= stream_k || (tm >= 128 && share < 12 && P != pieces)) cost = 1e9;
+    c[P - 2] = {cost, cost < 1e9 ? P : 0};
+  }
+  std::sort(c.begin(), c.end());
+  return {c[0].second, c[1].second, c[2].second};
+}
+
+template <int TM, int KS, bool GROUPED>
+int launch_tc2_few_tiles(const Problem &pr, int tiles, int k_iters, int pairs) {
+  if (!g_use_pair_cluster) return -2;
+  for (int P : pick_pair_clusters(TM, tiles, k_iters, pairs, problem_sm_count(pr))) {
+    const int rc = P == 2   ? launch_tc2_cluster<TM, KS, GROUPED, 2>(pr)
+                   : P == 3 ? launch_tc2_cluster<TM, KS, GROUPED, 3>(pr)
+                   : P == 4 ? launch_tc2_cluster<TM, KS, GROUPED, 4>(pr)
+                            : -2;
+    if (rc != -2) return rc;
+  }
+  return -2;
+}
+
 template <int TM, int KS, bool GROUPED, int OUT>
 int launch_tc2(const Problem &pr) {
   using Cfg = w4a16::Config2<TM, KS, OUT>;
@@ -749,6 +863,10 @@ int launch_tc2(const Problem &pr) {
   if (pairs < 1) pairs = 1;
   if (pairs > fit_pairs) pairs = fit_pairs;
   if (pairs > MAX_GRID / 2) pairs = MAX_GRID / 2;
+  if (p.n_tiles * p.m_tiles <= pairs && pr.sms <= 0 && g_aligned_cut) {
+    const int rc = launch_tc2_few_tiles<TM, KS, GROUPED>(pr, p.n_tiles * p.m_tiles, p.k_iters, pairs);
+    if (rc != -2) return rc;
+  }
   if (pairs > p.total_iters) pairs = p.total_iters;
   // With two or more tiles per pair, all but the last one or two are taken whole and round-robin (tiles in flight at
   // one time are neighbours and share their operands in L2); the rest is split by k-stages as before.

@@ -81,7 +81,7 @@ struct Params {
   int dp_waves, sk_tile0, workers, m_fast;
   const __half *s;                      // scales (read directly by the epilogue when per-channel)
   __half *C;
-  __half *C2;                           // null, or (OUT_DUAL, and the mma.sync kernel) where else the result goes, [m][n]
+  __half *C2;                           // null, or where else the result goes, [m][n] (OUT_DUAL; the mma.sync kernel and clusters of pairs)
   uint32_t *partials;                   // [gridDim.x][TM][128] fp32 partial tiles; PARTIAL_IDLE between launches
   int *status;                          // 0, or STATUS_TIMEOUT | (site << 8)
   uint64_t wait_ns;                     // every device-side wait gives up after this long (WAIT_LIMIT_NS by default)
@@ -238,6 +238,26 @@ static_assert(sizeof(Bars) <= 1024, "barrier block");
 // warp-collective).
 __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int *abort, uint64_t limit_ns) {
   const bool ok = sm100::mbar_wait(bar, parity, abort, limit_ns);
+  return __all_sync(0xffffffffu, ok);
+}
+
+// Waits for the bytes that st_async of other CTAs of the cluster counts; bounded, but not cut short by an abort: a CTA whose
+// neighbours may still send must not leave.
+__device__ __forceinline__ bool warp_wait_cluster(uint32_t bar, uint32_t parity, uint64_t limit_ns) {
+  const uint64_t t0 = sm100::globaltimer_ns();
+  bool ok = false;
+  for (uint32_t i = 1;; ++i) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    if ((ok = done != 0)) break;
+    if ((i & 0x3f) == 0 && sm100::globaltimer_ns() - t0 > limit_ns) break;
+  }
   return __all_sync(0xffffffffu, ok);
 }
 

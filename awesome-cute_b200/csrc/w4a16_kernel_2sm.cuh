@@ -19,8 +19,9 @@
 
 namespace w4a16 {
 
-template <int TM, int KS_ = 128, int OUT = OUT_PLAIN>
+template <int TM, int KS_ = 128, int OUT = OUT_PLAIN, int P = 1>
 struct Config2 {
+  static_assert(P == 1 || OUT == OUT_PLAIN, "the cluster form has one epilogue for every destination");
   static_assert(TM == 32 || TM == 64 || TM == 128 || TM == 192, "batch tile of the pair");
   static_assert(KS_ == 128 || KS_ == 256, "k per stage");
   static constexpr int KS = KS_;
@@ -41,12 +42,15 @@ struct Config2 {
   static constexpr int BAR_BYTES = 1024;
   static constexpr int GATHER_BYTES = staged_output(OUT) ? GATHER_SLAB_BYTES : 0;
   static constexpr int SMEM_MAX = 227 * 1024;
-  static constexpr int STAGES_RAW = (SMEM_MAX - BAR_BYTES - GATHER_BYTES - 1024) / STAGE_BYTES;
-  static constexpr int STAGES = STAGES_RAW > 8 ? 8 : STAGES_RAW;
+  // cluster form: the other pairs' partial sums of the 16-row chunks this pair finishes, [chunk / P][P - 1][16][128] fp32
+  static constexpr int CHUNKS = TM / 16;
+  static constexpr int XSLAB_BYTES = P > 1 ? (CHUNKS + P - 1) / P * (P - 1) * 16 * TILE_N * 4 : 0;
+  static constexpr int STAGES_RAW = (SMEM_MAX - BAR_BYTES - GATHER_BYTES - XSLAB_BYTES - 1024) / STAGE_BYTES;
+  static constexpr int STAGES = STAGES_RAW > 8 ? 8 : STAGES_RAW & ~1;   // even: a stage is always converted by the same set
   static_assert(STAGES >= 3, "ring too shallow");
   static constexpr int NSETS = 2, NDQ = 8;
   static constexpr int THREADS = (NDQ + EPI_WARPS + 2) * 32;
-  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + BAR_BYTES + GATHER_BYTES + 1024;
+  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + BAR_BYTES + GATHER_BYTES + XSLAB_BYTES + 1024;
 };
 
 struct Bars2 {  // same offsets in both CTAs of the pair
@@ -58,6 +62,7 @@ struct Bars2 {  // same offsets in both CTAs of the pair
   uint64_t accfull[2];   // accumulator complete (commit to both CTAs)                        (local)
   uint64_t accempty[2];  // accumulator drained by both CTAs' epilogue warps                  (used in the leader)
   uint64_t drain;
+  uint64_t xfull;        // cluster form: the other pairs' partial sums of this CTA's chunks have arrived     (local)
   uint64_t gfull[2];     // gathering epilogue: this CTA's four epilogue warps have staged a chunk     (local)
   uint32_t tmem_base;
   int abort;
@@ -70,12 +75,21 @@ static_assert(sizeof(Bars2) <= 1024, "barrier block");
 // so both stay in L2); with contiguous ranges alone the pairs are spread over the whole problem and a batch whose
 // activations exceed L2 is re-read from HBM for every tile.  The stream-K part at the end levels the last wave, as in
 // the reference's dense stream-K demo (gemm/streamk_gemm/dp_sk_block.h:82-173 splits full waves from the remainder).
+// Cluster form (P > 1): the pair's share of its cluster's one tile.
+template <int P>
 struct Walk {
   int dp_tile, stride, sk_tile0, it, it_end, k_iters;
   __device__ __forceinline__ Walk(const Params &p, int pair)
       : dp_tile(pair), stride(p.workers), sk_tile0(p.sk_tile0), k_iters(p.k_iters) {
-    it = min(p.total_iters, pair * p.iters_per_cta);
-    it_end = min(p.total_iters, it + p.iters_per_cta);
+    if (P > 1) {
+      const int tile = pair / P, kb = (pair - tile * P) * p.iters_per_cta;
+      dp_tile = 0, sk_tile0 = 0;
+      it = tile * k_iters + kb;
+      it_end = tile * k_iters + min(k_iters, kb + p.iters_per_cta);
+    } else {
+      it = min(p.total_iters, pair * p.iters_per_cta);
+      it_end = min(p.total_iters, it + p.iters_per_cta);
+    }
   }
   __device__ __forceinline__ bool next(int &tile, int &kb, int &ke) {
     if (dp_tile < sk_tile0) {
@@ -113,11 +127,16 @@ __device__ __forceinline__ int tile_width(const Params &p, int m0) {
   return max(16, (rows + 15) & ~15);
 }
 
-template <int TM, int KS_, bool GROUPED, int OUT = OUT_PLAIN>
+// P > 1: the cluster form for problems with few tiles.  A cluster of P pairs owns one tile and cuts its k-range P ways.  The
+// 16-row chunks of the tile are finished by the pairs in turn: every CTA sends its partial sums of the others' chunks (of its
+// own 128 columns) straight into their shared memory, each store counted on the receiver's barrier, adds what it
+// receives in the order of the k-ranges, and writes its chunks of C.  In the stream-K form one pair folds the others'
+// partial tiles of up to 192 rows through L2, sixteen rows a round trip, when everybody else is done.
+template <int TM, int KS_, bool GROUPED, int OUT = OUT_PLAIN, int P = 1>
 __global__ void __launch_bounds__(Config2<TM, KS_>::THREADS, 1)
 w4a16_tc2_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmA,
                  const __grid_constant__ CUtensorMap tmS, const __grid_constant__ CUtensorMap tmC, const Params p) {
-  using Cfg = Config2<TM, KS_, OUT>;
+  using Cfg = Config2<TM, KS_, OUT, P>;
   constexpr bool GATHER = OUT == OUT_GATHER;
   using namespace sm100;
   constexpr int S = Cfg::STAGES, NDQ = Cfg::NDQ, KS = Cfg::KS;
@@ -135,14 +154,14 @@ w4a16_tc2_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant_
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const uint32_t rank = cluster_ctarank();          // 0 = leader
+  const uint32_t crank = cluster_ctarank();
+  const uint32_t rank = crank & 1, leader = crank & ~1u;   // in the pair (0 = leader), cluster rank of the leader
   const int pair = blockIdx.x >> 1;
 
   // ---- the PAIR's share: dp_waves whole tiles, then its slice of the linearised (256-column tile, k-stage) space of
   // the stream-K part; p.n_tiles counts 256-column tiles
-  const int it_begin = min(p.total_iters, pair * p.iters_per_cta);
-  const int it_end = min(p.total_iters, it_begin + p.iters_per_cta);
-  const int nsteps = p.dp_waves * p.k_iters + (it_end - it_begin);
+  const Walk<P> share(p, pair);
+  const int nsteps = (P > 1 ? 0 : p.dp_waves * p.k_iters) + (share.it_end - share.it);
 
   auto issue_weights = [&](int st, int n_idx2, int kk) {   // this CTA's 128 columns of the pair's tile
     const uint32_t full = smem_u32(&bars->wsfull[st]);
@@ -152,7 +171,7 @@ w4a16_tc2_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant_
     if (GROUPED) tma_load_2d(smem_u32(sS) + st * Cfg::S_BYTES, &tmS, n_idx * TILE_N, kk * Cfg::GROUPS, full);
   };
   auto issue_acts = [&](int st, int m0, int kk) {          // this CTA's half of the activation rows
-    const uint32_t leader_full = map_to_cta(smem_u32(&bars->afull[st]), 0);
+    const uint32_t leader_full = map_to_cta(smem_u32(&bars->afull[st]), leader);
     if (rank == 0) mbar_expect_tx(smem_u32(&bars->afull[st]), 2 * Cfg::A_BYTES);
     tma_load_3d_pair(smem_u32(sA) + st * Cfg::A_BYTES, &tmA, 0, m0 + (int)rank * (tile_width<TM>(p, m0) >> 1), kk * Cfg::KCHUNKS, leader_full);
   };
@@ -174,9 +193,16 @@ w4a16_tc2_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant_
       mbar_init(smem_u32(&bars->gfull[i]), EPI_WARPS);
     }
     mbar_init(smem_u32(&bars->drain), 1);
+    mbar_init(smem_u32(&bars->xfull), 1);
     bars->abort = 0;
     mbar_fence_init();
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    if (P > 1) {   // what the other pairs will send: their sums of the chunks q, q + P, ... of this tile
+      int n_idx2, m_idx;
+      tile_nm(p, pair / P, n_idx2, m_idx);
+      const int chunks = tile_width<TM>(p, m_idx * TM) / 16, q = pair % P;
+      if (q < chunks) mbar_expect_tx(smem_u32(&bars->xfull), (uint32_t)((chunks - q + P - 1) / P * (P - 1) * 16 * TILE_N * 4));
+    }
   }
   if (warp == MMA_WARP) {          // one warp in EACH CTA of the pair, same warp index, same destination offset
     tmem_alloc_pair(smem_u32(&bars->tmem_base), Cfg::TMEM_COLS);
@@ -186,6 +212,70 @@ w4a16_tc2_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant_
   cluster_sync_all();              // both CTAs' barriers exist before anything can arrive on them
   tc_fence_after();
   const uint32_t tmem = __shfl_sync(0xffffffffu, bars->tmem_base, 0);
+
+  // Cluster form: this warp's part of the exchange and of the finished chunks; h of H warps per TMEM lane quadrant
+  auto exchange = [&](int h, int H) {
+    const int quad = warp & 3, row = quad * 32 + lane, q = pair % P;
+    int n_idx2, m_idx;
+    tile_nm(p, pair / P, n_idx2, m_idx);
+    const int n0 = (2 * n_idx2 + (int)rank) * TILE_N, m0 = m_idx * TM, width = tile_width<TM>(p, m0);
+    __half sch = __float2half(1.0f);
+    if (!GROUPED) {
+      const int c32 = row & 31;
+      sch = p.s[n0 + row - c32 + 8 * ((c32 & 7) >> 1) + 2 * (c32 >> 3) + (c32 & 1)];
+    }
+    pdl_wait_prior_grid();
+    if (!warp_wait(smem_u32(&bars->accfull[0]), 0, abort, p.wait_ns)) { give_up(p, abort, 13); return; }
+    tc_fence_after();
+    const uint32_t t_acc = tmem + ((uint32_t)(quad * 32) << 16);
+    float *slab = reinterpret_cast<float *>(reinterpret_cast<uint8_t *>(bars) + Cfg::BAR_BYTES + Cfg::GATHER_BYTES);
+    const uint32_t slab_u = smem_u32(slab) + (uint32_t)row * 4, bar_u = smem_u32(&bars->xfull);
+#pragma unroll 1
+    for (int c = h; c * 16 < width; c += H) {
+      const int owner = c % P;
+      if (owner == q) continue;
+      uint32_t v[16];
+      tmem_ld_32x32b_x16(t_acc + c * 16, v);
+      tc_wait_ld();
+      const uint32_t to = 2 * owner + rank, slot = (uint32_t)(c / P * (P - 1) + (q < owner ? q : q - 1));
+      const uint32_t dst = map_to_cta(slab_u + slot * (16 * TILE_N * 4), to), dbar = map_to_cta(bar_u, to);
+#pragma unroll
+      for (int i = 0; i < 16; ++i) st_async_f32(dst + (uint32_t)i * (TILE_N * 4), __uint_as_float(v[i]), dbar);
+    }
+    const int dests = 1 + p.n_extra + (p.C2 ? 1 : 0);
+    // (longer than any other wait: a CTA that gave up sends nothing, one that did not sends before this ends)
+    if (q * 16 < width && !warp_wait_cluster(bar_u, 0, 8 * p.wait_ns)) { give_up(p, abort, 14); return; }
+#pragma unroll 1
+    for (int c = h; c * 16 < width; c += H) {
+      if (c % P != q) continue;
+      uint32_t v[16];
+      tmem_ld_32x32b_x16(t_acc + c * 16, v);
+      tc_wait_ld();
+      float f[16];
+      const float *src = slab + c / P * (P - 1) * 16 * TILE_N + row;
+#pragma unroll
+      for (int o = 0; o < P; ++o) {   // in the order of the k-ranges
+        const float *part = src + (o < q ? o : o - 1) * 16 * TILE_N;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          const float x = o == q ? __uint_as_float(v[i]) : part[i * TILE_N];
+          f[i] = o == 0 ? x : f[i] + x;
+        }
+      }
+      // to C, and where the caller asks for it to host memory or the other ranks' buffers as well (plain stores)
+#pragma unroll 1
+      for (int d = 0; d < dests; ++d) {
+        __half *C = d == 0 ? p.C : d <= p.n_extra ? p.C_extra[d - 1] : p.C2;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          const int mm = m0 + c * 16 + i;
+          __half hv = __float2half(f[i]);
+          if (!GROUPED) hv = __hmul(hv, sch);  // per-channel scale after the fp16 convert (marlin_cute_trait.h:764-769)
+          if (mm < p.m) C[(size_t)mm * p.c_ld + p.c_col0 + n0 + row] = hv;
+        }
+      }
+    }
+  };
 
   if (warp < NDQ) {
     // =========================================================== dequant warps (as in the single-CTA kernel)
@@ -243,17 +333,19 @@ w4a16_tc2_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant_
       tc_fence_before();
       __syncwarp();
       if (lane == 0) {
-        mbar_arrive_cluster(map_to_cta(smem_u32(&bars->wfull[wb]), 0));   // the leader's MMA warp counts both CTAs
+        mbar_arrive_cluster(map_to_cta(smem_u32(&bars->wfull[wb]), leader));   // the leader's MMA warp counts both CTAs
         mbar_arrive(smem_u32(&bars->empty[st]));
       }
       d_work += W4A16_CLK() - c1;
     }
     if (warp == 0) { W4A16_BUCKET(4, d_full); W4A16_BUCKET(5, d_wempty); W4A16_BUCKET(6, d_work); }
-    if (HELP) {
+    if (P > 1) {
+      if (HELP) exchange(1 + set, 1 + Cfg::NSETS);
+    } else if (HELP) {
       // ---- help to finish the CTA's last tile if it is a split one (chunks 16*(1+set), +48, ... of this quadrant)
       int l_tile = 0, l_kb = 1, l_ke = 0, l_seg = -1;
       {
-        Walk walk(p, pair);
+        Walk<P> walk(p, pair);
         int t, kb, ke;
         while (walk.next(t, kb, ke)) l_tile = t, l_kb = kb, l_ke = ke, ++l_seg;
       }
@@ -293,6 +385,8 @@ w4a16_tc2_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant_
         if (!ok) give_up(p, abort, 19);
       }
     }
+  } else if (P > 1 && warp < NDQ + EPI_WARPS) {
+    exchange(0, HELP ? 1 + Cfg::NSETS : 1);
   } else if (warp < NDQ + EPI_WARPS) {
     // =========================================================== epilogue warps: this CTA's 128 columns, all TM rows
     const int quad = warp & 3;
@@ -301,7 +395,7 @@ w4a16_tc2_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant_
     pdl_wait_prior_grid();
     __half *slabs = reinterpret_cast<__half *>(reinterpret_cast<uint8_t *>(bars) + Cfg::BAR_BYTES);   // gathering form only
     int gcount = 0;
-    Walk walk(p, pair);
+    Walk<P> walk(p, pair);
     int tile, kb, ke;
     for (int seg = 0; walk.next(tile, kb, ke); ++seg) {
       int n_idx2, m_idx;
@@ -360,7 +454,7 @@ w4a16_tc2_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant_
       if (!ok) { give_up(p, abort, 14); break; }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&bars->accempty[acc]), 0));
+      if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&bars->accempty[acc]), leader));
     }
     // the TMA stores of this thread have left shared memory and reached C before the CTA ends (also after a give-up)
     if (OUT == OUT_TMA && quad == 0 && lane == 0) tma_store_wait_all();
@@ -370,7 +464,7 @@ w4a16_tc2_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant_
     const int first = min(S, nsteps);
     int step = 0;
     {  // weights of the first ring-full: parameters, requested before the previous kernel of the stream is known done
-      Walk walk(p, pair);
+      Walk<P> walk(p, pair);
       int tile, kb, ke, i = 0;
       while (i < first && walk.next(tile, kb, ke)) {
         int n_idx2, m_idx;
@@ -384,7 +478,7 @@ w4a16_tc2_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant_
     pdl_launch_dependents();
     pdl_wait_prior_grid();
     {
-      Walk walk(p, pair);
+      Walk<P> walk(p, pair);
       int tile, kb, ke;
       bool ok = true;
       while (ok && walk.next(tile, kb, ke)) {
@@ -418,7 +512,8 @@ w4a16_tc2_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant_
     bool ok = true;
     long long m_afull = 0, m_wfull = 0, m_issue = 0, m_acc = 0;
     const uint32_t sA_u = smem_u32(sA);
-    Walk walk(p, pair);
+    const uint16_t pair_mask = (uint16_t)(3u << leader);
+    Walk<P> walk(p, pair);
     int tile, kb, ke;
     for (; ok && walk.next(tile, kb, ke); ++seg) {
       int n_idx2, m_idx;
@@ -448,19 +543,19 @@ w4a16_tc2_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant_
             const uint64_t bd = b_desc + (uint64_t)(((q >> 2) * (Cfg::HALF_ROWS * 128) + (q & 3) * 32) >> 4);
             tc_mma_ts_pair(d_tmem, a_tmem + q * 8, bd, idesc, (kk > kb || q > 0) ? 1u : 0u);
           }
-          tc_commit_pair(smem_u32(&bars->wempty[wb]));
-          tc_commit_pair(smem_u32(&bars->empty[st]));
+          tc_commit_pair(smem_u32(&bars->wempty[wb]), pair_mask);
+          tc_commit_pair(smem_u32(&bars->empty[st]), pair_mask);
         }
         __syncwarp();
         m_issue += W4A16_CLK() - c2;
       }
-      if (ok && elect_one()) tc_commit_pair(smem_u32(&bars->accfull[acc]));
+      if (ok && elect_one()) tc_commit_pair(smem_u32(&bars->accfull[acc]), pair_mask);
       __syncwarp();
     }
     W4A16_BUCKET(8, m_afull); W4A16_BUCKET(9, m_wfull); W4A16_BUCKET(10, m_issue); W4A16_BUCKET(11, m_acc); W4A16_BUCKET(3, step);
     if (!ok || *abort) {   // unwinding: no MMA may still be running when tensor memory is freed
       volatile int never = 0;
-      if (elect_one()) tc_commit_pair(smem_u32(&bars->drain));
+      if (elect_one()) tc_commit_pair(smem_u32(&bars->drain), pair_mask);
       __syncwarp();
       mbar_wait(smem_u32(&bars->drain), 0, &never, 200000000ull);
     }

@@ -81,31 +81,6 @@ __device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], uint32_t addr) {
 __device__ __forceinline__ void lds128(uint32_t (&v)[4], uint32_t addr) {
   asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(addr) : "memory");
 }
-// 16 bytes into another CTA's shared memory, counted there on `bar`: data and signal in one, no fence on either side
-__device__ __forceinline__ void st_async_f4(uint32_t cluster_addr, float4 v, uint32_t cluster_bar) {
-  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(cluster_addr),
-               "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w), "r"(cluster_bar)
-               : "memory");
-}
-// waits for bytes that st_async_f4 of other CTAs of the cluster counts
-__device__ __forceinline__ bool warp_wait_cluster(uint32_t bar, uint32_t parity, uint64_t limit_ns) {
-  const uint64_t t0 = sm100::globaltimer_ns();
-  bool ok = false;
-  for (uint32_t i = 1;; ++i) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(done)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    if ((ok = done != 0)) break;
-    if ((i & 0x3f) == 0 && sm100::globaltimer_ns() - t0 > limit_ns) break;
-  }
-  return __all_sync(0xffffffffu, ok);
-}
-
 // Four neighbouring cells of a partial-tile slot: each cell is its own flag (idle or written), so the vector access need
 // not be atomic as a whole.
 __device__ __forceinline__ void st_slot4(uint32_t *p, float4 v) {

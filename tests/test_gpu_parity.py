@@ -452,6 +452,23 @@ def test_device_quantize_pack_edges(n, k, groupsize):
     assert np.array_equal(sp_dev.cpu().numpy().view(np.uint16), sp_host.view(np.uint16))
 
 
+@pytest.mark.parametrize("m,n,k,groupsize", [
+    (17, 512, 1024, 128), (33, 1024, 8192, -1), (64, 512, 768, 128), (40, 2048, 2816, 128), (24, 4096, 4096, -1),   # 256-k stages
+    (77, 5120, 5504, -1), (80, 1024, 2048, 128), (129, 512, 8192, 128), (190, 256, 1536, 128), (500, 512, 6272, -1), (100, 2048, 8192, 128)])
+def test_clusters_of_cta_pairs(m, n, k, groupsize):
+    """Few tiles: two, three and four pairs per tile, even and uneven shares of k, fewer 16-row chunks than pairs, ragged
+    batches, one and several batch tiles."""
+    assert pkg.plan(m, n, k, groupsize)[1]["kernel"] == "pairs"
+    A, q, s = orc.make_problem(m, n, k, groupsize, seed=m + n + k)
+    At, Bt, st = pack_problem(A, q, s)
+    C = run_mul(At, Bt, st, m, n)
+    for _ in range(3):
+        assert torch.equal(C, run_mul(At, Bt, st, m, n))
+    cols = np.r_[0:128, n - 128:n] if n * k > 1 << 22 else np.arange(n)     # oracle on the first and last columns only
+    ref = orc.c_gemm(A, np.ascontiguousarray(q[:, cols]), np.ascontiguousarray(s[:, cols]), groupsize)
+    check(C[:, torch.from_numpy(cols).to(C.device)], ref, "m=%d n=%d k=%d g=%d" % (m, n, k, groupsize))
+
+
 @pytest.mark.parametrize("m", [1, 8, 13, 40, 96])
 @pytest.mark.parametrize("shared", [False, True])
 def test_host_calls_in_a_chain(m, shared):
