@@ -522,7 +522,7 @@ int launch_decode_cluster(const Problem &pr) {
 // W4A16_TMA_STORE=0 / 1 in the environment picks how finished tiles of the plain GEMM reach C: 2-byte stores from
 // registers, or staged in shared memory and stored by the copy engine (cp.async.bulk.tensor).  Both are compiled
 // and tested; the default is the one measured faster (see tma_store_default).  The mma.sync kernel and
-// the clusters of CTA pairs have one form each.
+// the cluster forms always store from registers.
 const int g_tma_store = [] {
   const char *e = std::getenv("W4A16_TMA_STORE");
   return (e && (e[0] == '0' || e[0] == '1')) ? e[0] - '0' : -1;
@@ -544,8 +544,7 @@ int launch_decode_cluster_o(const Problem &pr, int cl) {
   return -2;
 }
 int launch_decode_cluster_g(const Problem &pr, int cl) {
-  if (pr.C2) return launch_decode_cluster_o<w4a16::OUT_DUAL>(pr, cl);
-  return use_tma_store(pr) ? launch_decode_cluster_o<w4a16::OUT_TMA>(pr, cl) : launch_decode_cluster_o<w4a16::OUT_PLAIN>(pr, cl);
+  return pr.C2 ? launch_decode_cluster_o<w4a16::OUT_DUAL>(pr, cl) : launch_decode_cluster_o<w4a16::OUT_PLAIN>(pr, cl);
 }
 
 // ---- up to 8 rows, and some of up to 16, on CTAs of half an SM: see w4a16_kernel_skinny.cuh

@@ -61,13 +61,14 @@ struct DecodeConfig {
   static constexpr int BAR_BYTES = 1024;
   // output staging: two padded slabs for the gathering epilogue, one 4 KB slab for the TMA store (a tile is one chunk)
   static constexpr int GATHER_BYTES = OUT == OUT_GATHER ? GATHER_SLAB_BYTES : OUT == OUT_TMA ? 2 * 16 * TILE_N * 2 : 0;
-  // cluster form: the other ranks' fp32 partial tiles land here, in rank 0's shared memory: [CL - 1][TM][128] fp32
-  static constexpr int XSLAB_BYTES = (CL - 1) * TM * TILE_N * 4;
+  // cluster form: the other ranks' partial sums of the rows this rank finishes, [TM / CL][CL - 1][128] fp32
+  static constexpr int XSLAB_BYTES = TM / CL * (CL - 1) * TILE_N * 4;
   static constexpr int SMEM_MAX = 227 * 1024;
   static constexpr int STAGES_RAW = (SMEM_MAX - BAR_BYTES - GATHER_BYTES - XSLAB_BYTES - 1024) / STAGE_BYTES;
-  // a multiple of the number of dequant sets, so that a stage is always converted by the same set; in the cluster
-  // form a CTA runs few stages and six are plenty
-  static constexpr int STAGES = CL > 1 ? 6 : (STAGES_RAW > 12 ? 12 : STAGES_RAW);
+  // Nine, or what fits: a ring of six in the cluster form costs 3-5 % where a rank has more stages than that (16 x 8192 x 8192
+  // 10.4 against 11.0 us).  A slot may be converted by different sets in turn: the epilogue folds the stages in order, so a
+  // set that has come to a stage knows that the one before it in the slot has been consumed.
+  static constexpr int STAGES = STAGES_RAW > 9 ? 9 : STAGES_RAW;
   static_assert(STAGES <= STAGES_RAW, "shared memory budget");
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + BAR_BYTES + GATHER_BYTES + XSLAB_BYTES + 1024 /*align slack*/;
 };
@@ -82,16 +83,18 @@ struct DecodeBars {  // lives in shared memory
   uint64_t accempty[4];
   uint64_t drain[4];     // one per MMA issuer warp
   uint64_t gfull[2];
+  uint64_t xfull;        // cluster form: the other ranks' rows have arrived
   uint32_t tmem_base;
   int abort;
 };
 static_assert(sizeof(DecodeBars) <= 1024, "barrier block");
 
 // CL > 1: the cluster form for layers with few tiles.  A cluster of CL CTAs (launched with that cluster dimension) owns
-// one tile and cuts its k-range CL ways; ranks 1.. send their fp32 partial tile straight into rank 0's shared memory
-// (st.shared::cluster; the data is its own flag, as in the stream-K fix-up), and rank 0 adds them in rank order and writes C.  The stream-K
-// form's fix-up goes through L2 instead, and when all CTAs of a tile finish together (which they do when a tile is cut
-// evenly) that costs the finisher two L2 round trips after everybody else is done; inside a cluster it is one hop.
+// one tile and cuts its k-range CL ways.  Rank r finishes the batch rows r, r + CL, ...: every rank sends its partial sums of
+// the others' rows straight into their shared memory (st.async: each store counts its bytes on the receiver's barrier, so
+// there is no release, no flag and no polling of data), adds what it receives in rank order and writes its rows of C.  The
+// stream-K form's fix-up goes through L2 instead, and when all CTAs of a tile finish together (which they do when a tile
+// is cut evenly) that costs the finisher two L2 round trips after everybody else is done; inside a cluster it is one hop.
 template <bool GROUPED, int OUT = OUT_PLAIN, int CL = 1>
 __global__ void __launch_bounds__(DecodeConfig<>::THREADS, 1)
 w4a16_decode_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmA,
@@ -171,6 +174,7 @@ w4a16_decode_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_consta
       mbar_init(smem_u32(&bars->gfull[lane - S - Cfg::WBUFS - Cfg::NACC]), EPI_WARPS);
     } else if (lane == 31) {
       for (int i = 0; i < Cfg::NMMA; ++i) mbar_init(smem_u32(&bars->drain[i]), 1);
+      mbar_init(smem_u32(&bars->xfull), 1);
       bars->abort = 0;
       tma_prefetch_desc(&tmB);
       tma_prefetch_desc(&tmS);
@@ -179,6 +183,10 @@ w4a16_decode_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_consta
     mbar_fence_init();
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncwarp();
+    if (CL > 1 && lane == 31) {   // the rows this rank finishes, from each of the other ranks
+      const int rows = (int)crank < p.m ? (p.m - (int)crank + CL - 1) / CL : 0;
+      if (rows) mbar_expect_tx(smem_u32(&bars->xfull), (uint32_t)(rows * (CL - 1) * TILE_N * 4));
+    }
     const int pro_tile = it_begin / p.k_iters;
     pro_kk = it_begin - pro_tile * p.k_iters;
     pro_nidx = pro_tile % p.n_tiles;
@@ -203,23 +211,10 @@ w4a16_decode_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_consta
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  // Cluster form: rank 0's slab must hold the idle pattern before another rank writes into it.  Every thread arrives
-  // at the cluster barrier here and waits for it only where it needs the guarantee (the epilogue threads of ranks 1..
-  // right before they send, everybody else at the end): waiting here held every warp for about a microsecond.
-  bool cluster_waited = false;
+  // Cluster form: every thread arrives here (the barriers' initialisation was released by fence.mbarrier_init) and waits
+  // only where it needs the other ranks: the epilogue warps right before they send, everybody else at the end.
   if (warp == 0) W4A16_STAMP(15);  // CTA-wide sync passed
-  if constexpr (CL > 1) {
-    if (crank == 0 && warp >= NDQ && warp < NDQ + EPI_WARPS) {
-      // rank 0's epilogue warps, idle for the next microseconds, put the idle pattern into the slab; their arrive
-      // releases it at cluster scope (that release is what costs ~1500 clocks: nobody else pays it)
-      uint32_t *cell = reinterpret_cast<uint32_t *>(reinterpret_cast<uint8_t *>(bars) + Cfg::BAR_BYTES + Cfg::GATHER_BYTES) + (warp - NDQ) * 32 + lane;
-#pragma unroll 4
-      for (int i = 0; i < (CL - 1) * TM; ++i) cell[(size_t)i * TILE_N] = PARTIAL_IDLE;
-      cluster_arrive();
-    } else {
-      cluster_arrive_relaxed();
-    }
-  }
+  if constexpr (CL > 1) cluster_arrive_relaxed();
   if (warp == 0) W4A16_STAMP(1);   // prologue done
   const uint32_t tmem = __shfl_sync(0xffffffffu, bars->tmem_base, 0);  // provably warp-uniform
 
@@ -319,7 +314,7 @@ w4a16_decode_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_consta
       const int last_contrib = (finisher && ke < p.k_iters) ? ((tile + 1) * p.k_iters - 1) / p.iters_per_cta : (int)blockIdx.x;
       const int ncontrib = last_contrib - (int)blockIdx.x;
       __half sch = __float2half(1.0f);
-      if (!GROUPED && finisher) {
+      if (!GROUPED && (CL > 1 || finisher)) {
         const int c32 = row & 31;  // per-channel scales are permuted inside 32-column blocks (marlin.py:52-54)
         sch = p.s[n0 + row - c32 + 8 * ((c32 & 7) >> 1) + 2 * (c32 >> 3) + (c32 & 1)];
       }
@@ -362,49 +357,47 @@ w4a16_decode_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_consta
         }
         if (warp == NDQ && step == 0) W4A16_STAMP(5);   // first accumulator folded
       }
-      if (!ok) break;
+      if (CL == 1 && !ok) break;
       if (warp == NDQ) W4A16_STAMP(6);                 // (last value wins) last accumulator folded
+      if constexpr (CL > 1) {
+        // Row i goes to rank i % CL, slot [i / CL][sender, without the receiver itself]; slab rows are 128 consecutive
+        // columns, so a warp's 4-byte stores are one 128-byte packet.
+        cluster_wait();
+        const uint32_t slab_u = smem_u32(xslab) + (uint32_t)row * 4, bar_u = smem_u32(&bars->xfull);
+        if (ok) {
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            const uint32_t owner = i % CL;
+            if (owner == crank || i >= p.m) continue;
+            const uint32_t slot = (i / CL) * (CL - 1) + (crank < owner ? crank : crank - 1);
+            st_async_f32(map_to_cta(slab_u + slot * (TILE_N * 4), owner), f[i], map_to_cta(bar_u, owner));
+          }
+        }
+        // A rank stays until its rows are complete, also after an abort: nothing may arrive in a CTA that has left.
+        // (Longer than any other wait: a rank that gave up sends nothing, one that did not sends before this ends.)
+        if ((int)crank < p.m && !warp_wait_cluster(bar_u, 0, 8 * p.wait_ns)) { give_up(p, abort, 4); ok = false; }
+        if (!ok) break;
+        if (warp == NDQ) W4A16_STAMP(7);               // partial rows arrived
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          if (i % CL != (int)crank || i >= p.m) continue;
+          const float own = f[i];
+          f[i] = 0.f;
+#pragma unroll
+          for (int o = 0; o < CL; ++o)   // in rank order
+            f[i] += o == (int)crank ? own : xslab[((i / CL) * (CL - 1) + (o < (int)crank ? o : o - 1)) * TILE_N + row];
+        }
+      }
       uint32_t v[16];
 #pragma unroll
       for (int i = 0; i < 16; ++i) v[i] = __float_as_uint(f[i]);
-      if (CL > 1 && !finisher) {
-        // cluster form, ranks 1..: the partial tile goes into rank 0's slab [rank - 1][16][128], one hop over the
-        // cluster's shared-memory network.  As in the stream-K form the data is its own flag (a cell is written when
-        // it no longer holds the idle pattern): a release at cluster scope would cost the sender ~1500 clocks.
-        // (Slab rows are 128 consecutive columns, so a warp's 4-byte stores are one 128-byte packet; a column-major
-        // slab written with 16-byte stores per thread was measured 4-7 % slower on every cluster shape.)
-        const uint32_t dst = map_to_cta(smem_u32(xslab + ((size_t)(crank - 1) * TM) * TILE_N + row), 0);
-        if (!cluster_waited) { cluster_wait(); cluster_waited = true; }
-#pragma unroll
-        for (int i = 0; i < 16; ++i) st_shared_cluster_u32(dst + (uint32_t)i * TILE_N * 4, v[i] == PARTIAL_IDLE ? 0x7fffffffu : v[i]);
-      } else if (!finisher) {
+      if (CL == 1 && !finisher) {
         // the data is its own flag: anything but the idle pattern means "written"
         uint32_t *part = p.partials + ((size_t)blockIdx.x * TM) * TILE_N + row;
 #pragma unroll
         for (int i = 0; i < 16; ++i) st_slot(part + (size_t)i * TILE_N, v[i] == PARTIAL_IDLE ? 0x7fffffffu : v[i]);
       } else {
-        if constexpr (CL > 1) {
-          // rank 0: re-read its own slab until no cell shows the idle pattern, then add in rank order
-          const uint32_t cell0 = smem_u32(xslab) + (uint32_t)row * 4;
-          const uint64_t t0 = globaltimer_ns();
-          for (uint32_t spin = 0;; ++spin) {
-            bool up = true;
-#pragma unroll 1
-            for (int r = 0; r < CL - 1; ++r)
-#pragma unroll
-              for (int i = 0; i < TM; ++i) up &= (ld_shared_relaxed_cluster(cell0 + (uint32_t)((r * TM + i) * TILE_N * 4)) != PARTIAL_IDLE);
-            if (__all_sync(0xffffffffu, up)) break;
-            if ((spin & 0x3f) == 0x3f && __any_sync(0xffffffffu, *abort || globaltimer_ns() - t0 > p.wait_ns)) { ok = false; break; }
-          }
-          if (!ok) { give_up(p, abort, 4); break; }
-#pragma unroll 1
-          for (int r = 0; r < CL - 1; ++r)
-#pragma unroll
-            for (int i = 0; i < 16; ++i) f[i] += __uint_as_float(ld_shared_relaxed_cluster(cell0 + (uint32_t)((r * TM + i) * TILE_N * 4)));
-#pragma unroll
-          for (int i = 0; i < 16; ++i) v[i] = __float_as_uint(f[i]);
-          if (warp == NDQ) W4A16_STAMP(7);             // partial tiles folded in
-        } else if (ncontrib > 0) {
+        if (CL == 1 && ncontrib > 0) {
           const uint64_t t0 = globaltimer_ns();
           if (!fold_partial_slices_call<3>(v, p.partials, TM, 0, row, (int)blockIdx.x + 1, 1, ncontrib, abort, t0, p.wait_ns)) {
             give_up(p, abort, 4);
@@ -419,7 +412,7 @@ w4a16_decode_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_consta
             ok = false;
             break;
           }
-        } else if constexpr (OUT == OUT_TMA) {
+        } else if constexpr (OUT == OUT_TMA && CL == 1) {
           if (!store_chunk_tma<GROUPED>(p, &tmC, v, sch, m0, n0, quad, lane, slabs, smem_u32(&bars->gfull[0]), gcount, abort)) {
             give_up(p, abort, 4);
             ok = false;
@@ -428,6 +421,7 @@ w4a16_decode_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_consta
         } else {
 #pragma unroll
           for (int i = 0; i < 16; ++i) {
+            if (CL > 1 && i % CL != (int)crank) continue;
             const int mm = m0 + i;
             __half hv = __float2half(__uint_as_float(v[i]));
             if (!GROUPED) hv = __hmul(hv, sch);  // per-channel scale after the fp16 convert (marlin_cute_trait.h:764-769)
@@ -577,11 +571,8 @@ w4a16_decode_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_consta
     tmem_dealloc(tmem, Cfg::TMEM_COLS);
     W4A16_STAMP(13);                       // TMEM freed
   }
-  // cluster form: rank 0's shared memory must outlive every store the other ranks may still send into it (they send
-  // only on the regular path, microseconds before this point; after a time-out nobody sends)
-  if constexpr (CL > 1) {
-    if (!cluster_waited) cluster_wait();
-    cluster_sync_all();
+  if constexpr (CL > 1) {   // (the epilogue warps have waited; every rank arrived in its prologue)
+    if (warp < NDQ || warp >= NDQ + EPI_WARPS) cluster_wait();
   }
 }
 
