@@ -155,13 +155,20 @@ w4a16_tc2_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant_
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const uint32_t crank = cluster_ctarank();
-  const uint32_t rank = crank & 1, leader = crank & ~1u;   // in the pair (0 = leader), cluster rank of the leader
+  const uint32_t rank = P == 1 ? crank : crank & 1;        // in the pair (0 = leader)
+  const uint32_t leader = P == 1 ? 0 : crank & ~1u;        // cluster rank of the leader
   const int pair = blockIdx.x >> 1;
 
   // ---- the PAIR's share: dp_waves whole tiles, then its slice of the linearised (256-column tile, k-stage) space of
   // the stream-K part; p.n_tiles counts 256-column tiles
-  const Walk<P> share(p, pair);
-  const int nsteps = (P > 1 ? 0 : p.dp_waves * p.k_iters) + (share.it_end - share.it);
+  int nsteps;
+  if constexpr (P > 1) {
+    const Walk<P> share(p, pair);
+    nsteps = share.it_end - share.it;
+  } else {
+    const int it_begin = min(p.total_iters, pair * p.iters_per_cta);
+    nsteps = p.dp_waves * p.k_iters + (min(p.total_iters, it_begin + p.iters_per_cta) - it_begin);
+  }
 
   auto issue_weights = [&](int st, int n_idx2, int kk) {   // this CTA's 128 columns of the pair's tile
     const uint32_t full = smem_u32(&bars->wsfull[st]);
@@ -193,7 +200,7 @@ w4a16_tc2_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant_
       mbar_init(smem_u32(&bars->gfull[i]), EPI_WARPS);
     }
     mbar_init(smem_u32(&bars->drain), 1);
-    mbar_init(smem_u32(&bars->xfull), 1);
+    if (P > 1) mbar_init(smem_u32(&bars->xfull), 1);
     bars->abort = 0;
     mbar_fence_init();
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -512,7 +519,7 @@ w4a16_tc2_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant_
     bool ok = true;
     long long m_afull = 0, m_wfull = 0, m_issue = 0, m_acc = 0;
     const uint32_t sA_u = smem_u32(sA);
-    const uint16_t pair_mask = (uint16_t)(3u << leader);
+    const uint16_t pair_mask = P == 1 ? 3 : (uint16_t)(3u << leader);
     Walk<P> walk(p, pair);
     int tile, kb, ke;
     for (; ok && walk.next(tile, kb, ke); ++seg) {
