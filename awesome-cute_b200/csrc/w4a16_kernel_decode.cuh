@@ -65,10 +65,19 @@ struct DecodeConfig {
   static constexpr int XSLAB_BYTES = TM / CL * (CL - 1) * TILE_N * 4;
   static constexpr int SMEM_MAX = 227 * 1024;
   static constexpr int STAGES_RAW = (SMEM_MAX - BAR_BYTES - GATHER_BYTES - XSLAB_BYTES - 1024) / STAGE_BYTES;
-  // Nine, or what fits: a ring of six in the cluster form costs 3-5 % where a rank has more stages than that (16 x 8192 x 8192
-  // 10.4 against 11.0 us).  A slot may be converted by different sets in turn: the epilogue folds the stages in order, so a
-  // set that has come to a stage knows that the one before it in the slot has been consumed.
+  // Nine, or what fits (eight beside the slabs of the clusters of 4 and 8 and of the staged epilogues).
   static constexpr int STAGES = STAGES_RAW > 9 ? 9 : STAGES_RAW;
+  // A parity wait is right only for a waiter that knows the barrier's phase before the awaited one to be over.  Where the
+  // number of stages is a multiple of the number of sets, a set comes back to the slots that it waited for itself.  Elsewhere
+  // the stage g - STAGES of the same slot was another set's.  Coming to stage g, a set knows through its own stage
+  // g - NSETS that the MMAs of g - NSETS - WBUFS have completed, hence that the epilogue, which takes the stages in order, had
+  // folded g - NSETS - WBUFS - NACC (= g - 9) and all before.  With fewer stages than that it waits for its operand buffer
+  // first (BUF_FIRST): then the MMAs of g - WBUFS have completed and all stages up to g - WBUFS - NACC are over.  (An issuer
+  // has waited at its own stage g - NMMA for the accumulator, for stages up to g - NMMA - NACC that is.)
+  // A ring of 8 with the buffer first against one of 6, us in a chain at 16 rows: 1024 x 28672 9.0 / 9.3, 2048 x 8192 6.0 / 6.2,
+  // 4096 x 11008 9.0 / 9.0; against 8 with the late wait: level.
+  static constexpr bool BUF_FIRST = STAGES % NSETS != 0 && STAGES < NSETS + WBUFS + NACC;
+  static_assert(STAGES % NSETS == 0 || STAGES >= WBUFS + NACC, "no wait may pass on an older phase of its barrier");
   static_assert(STAGES <= STAGES_RAW, "shared memory budget");
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + BAR_BYTES + GATHER_BYTES + XSLAB_BYTES + 1024 /*align slack*/;
 };
@@ -240,6 +249,11 @@ w4a16_decode_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_consta
     for (int g = set, use = 0; g < nsteps; g += Cfg::NSETS, ++use) {   // g: this CTA's running stage number
       const int st = g % S;
       const long long c0 = W4A16_CLK();
+      const bool buf_first = Cfg::BUF_FIRST && g >= S;   // (see BUF_FIRST)
+      if (buf_first) {
+        if (!warp_wait(wempty_bar, (use & 1) ^ 1, abort, p.wait_ns)) { give_up(p, abort, 2); break; }
+        tc_fence_after();
+      }
       if (!warp_wait(smem_u32(&bars->full[st]), (g / S) & 1, abort, p.wait_ns)) { give_up(p, abort, 1); break; }
       const long long c1 = W4A16_CLK();
       if (warp == 0 && g == 0) W4A16_STAMP(2);   // first stage landed
@@ -263,7 +277,7 @@ w4a16_decode_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_consta
             dequant_word<false>(w, unused, v[4 * rr], v[4 * rr + 2]);
             dequant_word<false>(w >> 8, unused, v[4 * rr + 1], v[4 * rr + 3]);
           }
-          if (h == 0 && jj == 0) {
+          if (h == 0 && jj == 0 && !buf_first) {
             // the operand buffer is needed only now: the first words were converted while the MMAs that last read
             // it were still running
             const long long c2 = W4A16_CLK();

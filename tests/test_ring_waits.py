@@ -1,0 +1,154 @@
+"""The kernels' barrier protocol in a host model: no wait may pass on an older phase of its barrier.
+
+An mbarrier wait names the parity of a phase, so it is right only for a waiter that knows the phase before to be over: a
+waiter that comes earlier passes at once and reads a slot whose data is not there.  The kernels' rings are walked by several
+warps in turn, and which depths are safe follows from what a warp has waited for before.  Here the roles run as coroutines over
+model barriers, with one copy held back as long as anything else can move; the depths are those that the kernels are
+compiled with (tests/cpp/ring_depths.cu)."""
+import os
+import random
+import subprocess
+
+import pytest
+
+import __graft_entry__ as entry
+
+PROGRAM = os.path.join(entry.ROOT, "tests", "cpp", "ring_depths")
+
+
+class Bar:
+    def __init__(self, count):
+        self.count = self.left = count
+        self.phase = 0
+
+    def arrive(self):
+        self.left -= 1
+        if self.left == 0:
+            self.left, self.phase = self.count, self.phase + 1
+
+    def passes(self, parity):       # mbarrier.try_wait.parity
+        return (self.phase & 1) != parity
+
+
+class Stale(Exception):
+    pass
+
+
+def run(kernel, c, nsteps, late, seed):
+    """One CTA over `nsteps` stages; `late` = (kind, stage) of the copy that lands last.  Raises Stale when a role reads a
+    slot that does not hold its stage, or when the roles wait for one another for good."""
+    rng = random.Random(seed)
+    S, sets, bufs = c["stages"], c["sets"], c["bufs"]
+    per_set = kernel == "decode"                # an issuer and an accumulator set behind each dequant set
+    full = [Bar(1) for _ in range(S)]
+    afull = [Bar(1) for _ in range(S)]
+    empty = [Bar(3 if per_set else 2) for _ in range(S)]
+    wfull, wempty = [Bar(1) for _ in range(bufs)], [Bar(1) for _ in range(bufs)]
+    accfull, accempty = [Bar(1) for _ in range(sets)], [Bar(1) for _ in range(sets)]
+    slot_w, slot_a, operand = [None] * S, [None] * S, [None] * bufs
+    copies, mmas = [], {}                       # in flight: copies in any order, one issuer's MMAs in theirs
+
+    def expect(have, want, what):
+        if have != want:
+            raise Stale("%s of stage %s read where stage %d is due" % (what, have, want))
+
+    def producer():
+        for g in range(nsteps):
+            if g >= S:
+                yield empty[g % S], (g // S & 1) ^ 1
+            copies.extend([("w", g), ("a", g)])
+
+    def dequant(s):
+        for g in range(s, nsteps, sets):
+            st, wb = g % S, g % bufs
+            first = c["buf_first"] and g >= S
+            if first:
+                yield wempty[wb], (g // bufs & 1) ^ 1
+            yield full[st], g // S & 1
+            expect(slot_w[st], g, "weights")
+            if not first:
+                yield wempty[wb], (g // bufs & 1) ^ 1
+            operand[wb] = g
+            wfull[wb].arrive()
+            empty[st].arrive()
+
+    def issuer(i, step):
+        for g in range(i, nsteps, step):
+            st, wb = g % S, g % bufs
+            yield afull[st], g // S & 1
+            yield wfull[wb], g // bufs & 1
+            yield accempty[g % sets], (g // sets & 1) ^ 1
+            expect(slot_a[st], g, "activations")
+            expect(operand[wb], g, "operand")
+            mmas.setdefault(i, []).append(g)
+
+    def epilogue():
+        for g in range(nsteps):
+            yield accfull[g % sets], g // sets & 1
+            accempty[g % sets].arrive()
+            empty[g % S].arrive()
+
+    def land(kind, g):
+        st = g % S
+        if kind == "w":
+            slot_w[st] = g
+            full[st].arrive()
+        else:
+            slot_a[st] = g
+            afull[st].arrive()
+
+    def complete(i):
+        g = mmas[i].pop(0)
+        for b in (accfull[g % sets], wempty[g % bufs], empty[g % S]):
+            b.arrive()
+
+    roles = [producer(), epilogue()] + [dequant(s) for s in range(sets)] + [issuer(i, sets) for i in range(sets)]
+    waits = {}
+    for r in roles:
+        waits[r] = next(r, None)
+    while any(w is not None for w in waits.values()):
+        moves = [("role", r) for r, w in waits.items() if w is not None and w[0].passes(w[1])]
+        moves += [("mma", i) for i in mmas if mmas[i]]
+        moves += [("copy", x) for x in copies if x != late]
+        if not moves:
+            if late not in copies:
+                raise Stale("every role waits")
+            moves = [("copy", late)]
+        what, x = rng.choice(moves)
+        if what == "role":
+            waits[x] = next(x, None)
+        elif what == "mma":
+            complete(x)
+        else:
+            copies.remove(x)
+            land(*x)
+
+
+def explore(kernel, c):
+    nsteps = 2 * c["stages"] + c["sets"] + 1
+    for kind in "wa":
+        for stage in range(c["stages"] + c["sets"]):
+            for seed in range(4):
+                run(kernel, c, nsteps, (kind, stage), seed)
+
+
+def depths():
+    if not os.path.exists(PROGRAM):
+        entry._make(os.path.dirname(PROGRAM))
+    out = subprocess.run([PROGRAM], capture_output=True, text=True, check=True).stdout
+    rows = [line.split() for line in out.splitlines()]
+    return [(r[0], {k: int(v) for k, v in (x.split("=") for x in r[1:])}) for r in rows]
+
+
+def test_no_wait_passes_on_an_older_phase():
+    rows = depths()
+    assert {r[0] for r in rows} == {"decode"} and len(rows) == 10
+    for kernel, c in rows:
+        explore(kernel, c)
+
+
+@pytest.mark.parametrize("stages,buf_first", [(8, 0), (7, 0), (5, 1)])
+def test_the_model_sees_the_race(stages, buf_first):
+    """Eight stages walked by three sets that do not wait for their operand buffer first; five that do."""
+    with pytest.raises(Stale):
+        explore("decode", {"stages": stages, "sets": 3, "bufs": 3, "buf_first": buf_first})
