@@ -215,6 +215,12 @@ struct Config {
   // Two sets measured best on B200: a third adds eligible warps (+5 % on the largest decode shapes) but
   // costs registers (spills at TM = 128) and start-up time on small ones.
   static constexpr int NSETS = 2;                            // dequant sets taking k-stages round-robin
+  // A parity wait is right only for a waiter that knows the barrier's phase before the awaited one to be over.  With an odd
+  // number of stages the stage g - STAGES of the same slot was the other set's.  Coming to stage g, a set knows through its
+  // own stage g - NSETS that the MMAs of g - NSETS - WBUFS, which complete in order, and so all stages before are over; with
+  // fewer stages than that it waits for its operand buffer first (BUF_FIRST), for all stages up to g - WBUFS that is.
+  static constexpr bool BUF_FIRST = STAGES % NSETS != 0 && STAGES < NSETS + WBUFS;
+  static_assert(SUBS == 1 && (STAGES % NSETS == 0 || STAGES >= WBUFS), "no wait may pass on an older phase of its barrier");
   static constexpr int NDQ = 4 * NSETS;                      // dequant warps: NSETS sets of four
   static constexpr int THREADS = (NDQ + EPI_WARPS + 2) * 32;
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + BAR_BYTES + GATHER_BYTES + 1024 /*align slack*/;
@@ -488,6 +494,11 @@ w4a16_tc_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant__
       const int step = g / Cfg::SUBS, sub = g % Cfg::SUBS;
       const int st = step % S, wb = g % Cfg::WBUFS;
       const long long c0 = W4A16_CLK();
+      const bool buf_first = Cfg::BUF_FIRST && step >= S;   // (see BUF_FIRST)
+      if (buf_first) {
+        if (!warp_wait(smem_u32(&bars->wempty[wb]), ((g / Cfg::WBUFS) & 1) ^ 1, abort, p.wait_ns)) { give_up(p, abort, 2); break; }
+        tc_fence_after();
+      }
       if (!warp_wait(smem_u32(&bars->full[st]), (step / S) & 1, abort, p.wait_ns)) { give_up(p, abort, 1); break; }
       const long long c1 = W4A16_CLK();
       if (warp == 0 && g == 0) W4A16_STAMP(2);   // first stage landed
@@ -513,7 +524,7 @@ w4a16_tc_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant__
             dequant_word<GROUPED>(w >> shift, sc, v[r * 8 + t], v[r * 8 + 4 + t]);
           }
         }
-        if (half == 0) {
+        if (half == 0 && !buf_first) {
           // the TMEM operand buffer is needed only now: the first chunk was converted while the MMA that
           // last read this buffer was still running
           const long long c2 = W4A16_CLK();

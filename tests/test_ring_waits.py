@@ -39,9 +39,11 @@ def run(kernel, c, nsteps, late, seed):
     slot that does not hold its stage, or when the roles wait for one another for good."""
     rng = random.Random(seed)
     S, sets, bufs = c["stages"], c["sets"], c["bufs"]
-    per_set = kernel == "decode"                # an issuer and an accumulator set behind each dequant set
-    full = [Bar(1) for _ in range(S)]
-    afull = [Bar(1) for _ in range(S)]
+    # decode: an issuer and an accumulator set behind each dequant set; elsewhere one issuer, and one accumulator for all of
+    # these stages.  general: weights and activations of a stage on one barrier.
+    per_set = kernel == "decode"
+    full = [Bar(2 if kernel == "general" else 1) for _ in range(S)]
+    afull = full if kernel == "general" else [Bar(1) for _ in range(S)]
     empty = [Bar(3 if per_set else 2) for _ in range(S)]
     wfull, wempty = [Bar(1) for _ in range(bufs)], [Bar(1) for _ in range(bufs)]
     accfull, accempty = [Bar(1) for _ in range(sets)], [Bar(1) for _ in range(sets)]
@@ -77,7 +79,8 @@ def run(kernel, c, nsteps, late, seed):
             st, wb = g % S, g % bufs
             yield afull[st], g // S & 1
             yield wfull[wb], g // bufs & 1
-            yield accempty[g % sets], (g // sets & 1) ^ 1
+            if per_set:
+                yield accempty[g % sets], (g // sets & 1) ^ 1
             expect(slot_a[st], g, "activations")
             expect(operand[wb], g, "operand")
             mmas.setdefault(i, []).append(g)
@@ -99,10 +102,13 @@ def run(kernel, c, nsteps, late, seed):
 
     def complete(i):
         g = mmas[i].pop(0)
-        for b in (accfull[g % sets], wempty[g % bufs], empty[g % S]):
+        for b in [wempty[g % bufs], empty[g % S]] + ([accfull[g % sets]] if per_set else []):
             b.arrive()
 
-    roles = [producer(), epilogue()] + [dequant(s) for s in range(sets)] + [issuer(i, sets) for i in range(sets)]
+    issuers = sets if per_set else 1
+    roles = [producer()] + [dequant(s) for s in range(sets)] + [issuer(i, issuers) for i in range(issuers)]
+    if per_set:
+        roles.append(epilogue())
     waits = {}
     for r in roles:
         waits[r] = next(r, None)
@@ -142,13 +148,15 @@ def depths():
 
 def test_no_wait_passes_on_an_older_phase():
     rows = depths()
-    assert {r[0] for r in rows} == {"decode"} and len(rows) == 10
-    for kernel, c in rows:
-        explore(kernel, c)
+    assert {r[0] for r in rows} == {"decode", "general", "pairs"} and len(rows) == 10 + 48 + 28
+    for kernel, c in {(k, tuple((x, c[x]) for x in ("stages", "sets", "bufs", "buf_first"))) for k, c in rows}:
+        explore(kernel, dict(c))
 
 
-@pytest.mark.parametrize("stages,buf_first", [(8, 0), (7, 0), (5, 1)])
-def test_the_model_sees_the_race(stages, buf_first):
-    """Eight stages walked by three sets that do not wait for their operand buffer first; five that do."""
+@pytest.mark.parametrize("kernel,stages,sets,bufs,buf_first", [
+    ("decode", 8, 3, 3, 0), ("decode", 7, 3, 3, 0), ("decode", 5, 3, 3, 1),
+    ("general", 5, 2, 4, 0), ("general", 3, 2, 2, 0), ("pairs", 5, 2, 4, 0)])
+def test_the_model_sees_the_race(kernel, stages, sets, bufs, buf_first):
+    """Rings whose depth is no multiple of the sets and too small for what a set knows."""
     with pytest.raises(Stale):
-        explore("decode", {"stages": stages, "sets": 3, "bufs": 3, "buf_first": buf_first})
+        explore(kernel, {"stages": stages, "sets": sets, "bufs": bufs, "buf_first": buf_first})
