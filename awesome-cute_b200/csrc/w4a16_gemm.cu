@@ -23,6 +23,7 @@
 
 #include "../../include/marlin_cute.h"
 #include "../../include/w4a16.h"
+#include "w4a16_host_chain.h"
 #include "w4a16_kernel.cuh"
 #include "w4a16_kernel_2sm.cuh"
 #include "w4a16_kernel_decode.cuh"
@@ -1192,9 +1193,9 @@ extern "C" int w4a16_plan(int prob_m, int prob_n, int prob_k, int groupsize, int
 //   * the GEMM's epilogue writes each result to C_stage and, over PCIe, to C_host.
 // The copy-in may run beside the previous calls' GEMMs when those are the last things this library has launched and neither
 // touches what the other writes; it ends only after the GEMM before it has, so whatever waits for a call has waited for
-// everything before it.  How many of the earlier calls may still be running then is bounded by nothing but the room on
-// the SMs, so their buffers are remembered since the last copy-in that waited first, eight calls at most.  (Any kernel of
-// other origin in between restores full stream order, unless it too lets its successor start early.)
+// everything before it.  Which calls may still be running then, and when a copy-in has to wait: w4a16_host_chain.h.  (Any
+// kernel of other origin in between restores full stream order, unless it too lets its successor start early; so does the
+// launch of a graph, whatever its kernels do.)
 // Several streams side by side overlap one call's copy engines with another's kernel, and there the SMs are worth more than the
 // latency (four layers on four streams 50 us with copy engines, 66 us without): the SMs copy when the last call of this
 // kind, by whatever thread, was on the same stream.  Four 7B layers at m = 16 in order on one stream: 159 -> 77 us (87-93
@@ -1210,10 +1211,11 @@ const int g_host_direct = [] {
 constexpr size_t HOST_COPY_MAX = 4u << 20;
 constexpr int COPY_THREADS = 1024, COPY_FLY = 4;
 
-// 16 bytes per thread and load, COPY_FLY loads in flight
-__global__ void __launch_bounds__(COPY_THREADS) copy_in_kernel(const uint4 *__restrict__ src, uint4 *__restrict__ dst, size_t n16, int early) {
-  sm100::pdl_launch_dependents();   // the GEMM behind this kernel orders itself with griddepcontrol.wait
-  if (!early) sm100::pdl_wait_prior_grid();
+// 16 bytes per thread and load, COPY_FLY loads in flight; the GEMM behind this kernel orders itself with griddepcontrol.wait
+__global__ void __launch_bounds__(COPY_THREADS) copy_in_kernel(const uint4 *__restrict__ src, uint4 *__restrict__ dst, size_t n16, int how) {
+  if (how == w4a16::COPY_FIRST) sm100::pdl_wait_prior_grid();
+  sm100::pdl_launch_dependents();
+  if (how == w4a16::COPY_LATE) sm100::pdl_wait_prior_grid();
   const size_t stride = (size_t)gridDim.x * COPY_THREADS;
   size_t i = (size_t)blockIdx.x * COPY_THREADS + threadIdx.x;
   for (; i + (COPY_FLY - 1) * stride < n16; i += COPY_FLY * stride) {
@@ -1242,27 +1244,9 @@ void *device_view_of_host(const void *host, size_t bytes) {
   return first.devicePointer;
 }
 
-bool overlap(const void *a, size_t na, const void *b, size_t nb) {
-  const uintptr_t x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b);
-  return x < y + nb && y < x + na;
-}
+w4a16::HostChain g_host_chain;   // guarded by g_mu
 
-// The last call with host buffers, and the buffers of all calls that may be unfinished when the next copy-in starts early:
-// those since the last copy-in that waited for everything before it (guarded by g_mu)
-struct HostBuffers {
-  const void *a_stage, *c_stage, *c_host;
-  size_t a_bytes, c_bytes;
-};
-struct HostChain {
-  bool any = false;
-  int dev = 0;
-  cudaStream_t stream = nullptr;
-  uint64_t launches = 0;                // g_launches after it, or 0 when its copies went through the copy engines
-  std::vector<HostBuffers> open;
-} g_host_chain;
-constexpr size_t HOST_CHAIN_MAX = 8;
-
-int launch_copy_in(const void *src, void *dst, size_t bytes, cudaStream_t st, int early) {
+int launch_copy_in(const void *src, void *dst, size_t bytes, cudaStream_t st, w4a16::CopyIn how) {
   cudaLaunchConfig_t cfg = {};
   // few SMs: one block per 64 KB, at most 16 (PCIe, not the SMs, bounds it), so that the GEMM's CTAs find theirs free
   cfg.gridDim = dim3((unsigned)std::min<size_t>(16, (bytes + 65535) / 65536));
@@ -1273,7 +1257,7 @@ int launch_copy_in(const void *src, void *dst, size_t bytes, cudaStream_t st, in
   attr[0].val.programmaticStreamSerializationAllowed = g_use_pdl ? 1 : 0;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cuda_ok(cudaLaunchKernelEx(&cfg, copy_in_kernel, static_cast<const uint4 *>(src), static_cast<uint4 *>(dst), bytes / 16, early),
+  return cuda_ok(cudaLaunchKernelEx(&cfg, copy_in_kernel, static_cast<const uint4 *>(src), static_cast<uint4 *>(dst), bytes / 16, (int)how),
                  "copy-in launch")
              ? W4A16_OK
              : W4A16_ERR_CUDA;
@@ -1293,18 +1277,14 @@ extern "C" int w4a16_marlin_gemm_host(const void *A_host, const void *B, void *C
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const size_t a_bytes = sizeof(__half) * (size_t)prob_m * prob_k, c_bytes = sizeof(__half) * (size_t)prob_m * prob_n;
 
+  const w4a16::HostBuffers bufs{A_host, A_stage, C_stage, C_host, a_bytes, c_bytes};
+
   bool direct = false;
-  int early = 0;
+  w4a16::CopyIn how = w4a16::COPY_FIRST;
   if (g_host_direct != 0 && a_bytes <= HOST_COPY_MAX && c_bytes <= HOST_COPY_MAX) {
     std::lock_guard<std::mutex> lock(g_mu);
-    const HostChain &l = g_host_chain;
-    const bool same = l.any && l.dev == dev && l.stream == st;
-    direct = g_host_direct == 1 || same;
-    early = direct && same && l.launches != 0 && l.launches == g_launches.load() && l.open.size() < HOST_CHAIN_MAX;
-    for (const HostBuffers &o : l.open)   // what this call's copy-in reads and writes
-      if (overlap(A_host, a_bytes, o.c_host, o.c_bytes) || overlap(A_stage, a_bytes, o.c_stage, o.c_bytes) ||
-          overlap(A_stage, a_bytes, o.a_stage, o.a_bytes))
-        early = 0;
+    direct = g_host_direct == 1 || g_host_chain.same_stream(dev, stream);
+    how = g_host_chain.order(dev, stream, g_launches.load(), bufs);
   }
   void *dA = nullptr, *dC = nullptr;
   if (direct) {
@@ -1315,23 +1295,20 @@ extern "C" int w4a16_marlin_gemm_host(const void *A_host, const void *B, void *C
   }
   int rc;
   if (direct)
-    rc = launch_copy_in(dA, A_stage, a_bytes, st, early);
+    rc = launch_copy_in(dA, A_stage, a_bytes, st, how);
   else
     rc = cuda_ok(cudaMemcpyAsync(A_stage, A_host, a_bytes, cudaMemcpyHostToDevice, st), "cudaMemcpyAsync(A)") ? W4A16_OK : W4A16_ERR_CUDA;
-  if (rc != W4A16_OK) return rc;
-  rc = gemm_entry(false, A_stage, B, C_stage, s, prob_m, prob_n, prob_k, workspace, groupsize, dev, st, -1, -1, sms, 16,
-                  direct ? dC : nullptr);
-  if (rc != W4A16_OK) return rc;
-  if (!direct && !cuda_ok(cudaMemcpyAsync(C_host, C_stage, c_bytes, cudaMemcpyDeviceToHost, st), "cudaMemcpyAsync(C)")) return W4A16_ERR_CUDA;
+  if (rc == W4A16_OK)
+    rc = gemm_entry(false, A_stage, B, C_stage, s, prob_m, prob_n, prob_k, workspace, groupsize, dev, st, -1, -1, sms, 16,
+                    direct ? dC : nullptr);
+  if (rc == W4A16_OK && !direct && !cuda_ok(cudaMemcpyAsync(C_host, C_stage, c_bytes, cudaMemcpyDeviceToHost, st), "cudaMemcpyAsync(C)"))
+    rc = W4A16_ERR_CUDA;
   std::lock_guard<std::mutex> lock(g_mu);
-  HostChain &l = g_host_chain;
-  l.any = true;
-  l.dev = dev;
-  l.stream = st;
-  l.launches = direct ? g_launches.load() : 0;
-  if (!early) l.open.clear();
-  l.open.push_back(HostBuffers{A_stage, C_stage, C_host, a_bytes, c_bytes});
-  return W4A16_OK;
+  if (rc == W4A16_OK)
+    g_host_chain.record(dev, stream, direct ? g_launches.load() : 0, direct ? how : w4a16::COPY_FIRST, bufs);
+  else
+    g_host_chain.forget();
+  return rc;
 }
 
 extern "C" int w4a16_marlin_gemm_simt(const void *A, const void *B, void *C, const void *s, int prob_m, int prob_n,

@@ -1,0 +1,66 @@
+// How the copy-in of a call with host buffers is ordered behind the calls before it (w4a16_marlin_gemm_host).  Host code
+// without CUDA, so that the rules can be checked on the CPU.
+//
+// Every kernel of this library waits for the completion of the one before it (griddepcontrol.wait) before it ends, so a kernel
+// that has waited has waited for everything before it.  But a GEMM lets its successor start (griddepcontrol.launch_dependents)
+// before it has waited itself, and the copy-in of COPY_EARLY and COPY_LATE does the same: what such a chain has in front of it
+// when it starts goes back, kernel by kernel, to the last one that waited FIRST, and all calls since then may be unfinished.
+// Those are the open calls.
+#pragma once
+#include <stddef.h>
+#include <stdint.h>
+
+#include <vector>
+
+namespace w4a16 {
+
+enum CopyIn {
+  COPY_FIRST = 0,   // waits, then lets the GEMM behind it start: everything before is over for all that follows
+  COPY_LATE = 1,    // lets the GEMM start (it prefetches its weights), waits, copies: shares a buffer with an open call
+  COPY_EARLY = 2,   // copies beside the open calls' GEMMs and waits at its end: shares none
+};
+
+struct HostBuffers {
+  const void *a_host, *a_stage, *c_stage, *c_host;
+  size_t a_bytes, c_bytes;
+};
+
+class HostChain {
+ public:
+  // The last call of this kind was on this stream.
+  bool same_stream(int dev, const void *stream) const { return any_ && dev_ == dev && stream_ == stream; }
+
+  // launches: the process's launch counter now
+  CopyIn order(int dev, const void *stream, uint64_t launches, const HostBuffers &b) const {
+    if (!same_stream(dev, stream) || launches_ == 0 || launches_ != launches || open_.size() >= MAX_OPEN) return COPY_FIRST;
+    for (const HostBuffers &o : open_)   // what the copy-in reads and writes
+      if (overlap(b.a_host, b.a_bytes, o.c_host, o.c_bytes) || overlap(b.a_stage, b.a_bytes, o.c_stage, o.c_bytes) ||
+          overlap(b.a_stage, b.a_bytes, o.a_stage, o.a_bytes))
+        return COPY_LATE;
+    return COPY_EARLY;
+  }
+
+  // After the call.  launches: the counter after it, or 0 when its copies went through the copy engines.
+  void record(int dev, const void *stream, uint64_t launches, CopyIn how, const HostBuffers &b) {
+    any_ = true, dev_ = dev, stream_ = stream, launches_ = launches;
+    if (how == COPY_FIRST) open_.clear();
+    open_.push_back(b);
+  }
+
+  // After a call that failed half-way: what it has launched is not known.
+  void forget() { launches_ = 0; }
+
+ private:
+  static bool overlap(const void *a, size_t na, const void *b, size_t nb) {
+    const uintptr_t x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b);
+    return x < y + nb && y < x + na;
+  }
+  static constexpr size_t MAX_OPEN = 8;
+  bool any_ = false;
+  int dev_ = 0;
+  const void *stream_ = nullptr;
+  uint64_t launches_ = 0;
+  std::vector<HostBuffers> open_;
+};
+
+}  // namespace w4a16

@@ -1,0 +1,17 @@
+// Test-only library: the ordering rules of host-buffer calls behind a C interface (loaded by tests/test_host_chain.py).
+#include "../../awesome-cute_b200/csrc/w4a16_host_chain.h"
+
+using w4a16::HostBuffers;
+using w4a16::HostChain;
+
+extern "C" {
+void *chain_new() { return new HostChain; }
+void chain_delete(void *c) { delete static_cast<HostChain *>(c); }
+int chain_order(void *c, int dev, const void *stream, uint64_t launches, const HostBuffers *b) {
+  return static_cast<HostChain *>(c)->order(dev, stream, launches, *b);
+}
+void chain_record(void *c, int dev, const void *stream, uint64_t launches, int how, const HostBuffers *b) {
+  static_cast<HostChain *>(c)->record(dev, stream, launches, static_cast<w4a16::CopyIn>(how), *b);
+}
+void chain_forget(void *c) { static_cast<HostChain *>(c)->forget(); }
+}

@@ -517,6 +517,48 @@ def test_host_calls_in_a_chain(m, shared):
     pkg.device_status(0)
 
 
+@pytest.mark.parametrize("m,d", [(1, 512), (8, 4096), (16, 4096), (40, 1024), (96, 2048)])
+def test_host_calls_that_share_buffers(m, d):
+    """Calls with host buffers, several passes without a synchronisation: two layers that read the same result, a staging
+    buffer that comes back after another call, a GEMM on a staging buffer that the next call fills, more calls than may
+    be unfinished at a time.  Every pass has inputs and host buffers of its own; results are those of mul() bit for bit."""
+    gen = torch.Generator(device=DEV).manual_seed(m + d)
+    Bs = [torch.randint(-2 ** 31, 2 ** 31, (d // 16, 2 * d), generator=gen, device=DEV, dtype=torch.int) for _ in range(6)]
+    s = (torch.rand((d // 128, d), generator=gen, device=DEV) * 0.1 + 0.95).mul_(0.2 * d ** -0.5).half()
+    ws = torch.zeros(d // 128 * 16, dtype=torch.int, device=DEV)
+    dev = lambda: torch.zeros((m, d), dtype=torch.half, device=DEV)
+    sa, sc = [dev() for _ in range(3)], [dev() for _ in range(3)]
+    stream = torch.cuda.Stream()
+    passes = []
+    for p in range(6):
+        h = [torch.zeros((m, d), dtype=torch.half).pin_memory() for _ in range(6)]
+        h[0].copy_(torch.randn((m, d), generator=gen, device=DEV).half())
+        op = lambda w, i, o, a, c: pkg.HostGemm(h[i], Bs[w], h[o], s, ws, sa[a], sc[c], stream=stream)
+        passes.append((h, dev(), [op(0, 0, 1, 0, 0), op(1, 1, 2, 1, 1), op(2, 1, 3, 0, 2), op(4, 0, 4, 1, 0), op(5, 4, 5, 2, 1)]))
+    torch.cuda.synchronize()
+    with torch.cuda.stream(stream):
+        for h, on_device, ops in passes:
+            for op in ops[:3]:
+                op()
+            pkg.mul(sa[1], Bs[3], on_device, s, ws)
+            for op in ops[3:]:
+                op()
+    stream.synchronize()
+    pkg.device_status(0)
+
+    def mul(a, w):
+        c = dev()
+        pkg.mul(a.to(DEV), Bs[w], c, s, ws)
+        return c
+
+    for h, on_device, _ in passes:
+        first = mul(h[0], 0)
+        assert torch.equal(h[1], first.cpu())
+        for have, want in ((h[2], mul(first, 1)), (h[3], mul(first, 2)), (on_device, mul(first, 3)), (h[4], mul(h[0], 4))):
+            assert torch.equal(have.to(DEV), want)
+        assert torch.equal(h[5].to(DEV), mul(h[4], 5))
+
+
 @pytest.mark.parametrize("n,k", [(128, 128), (256, 512), (128, 11008), (4096, 4096), (8192, 8192), (1280, 4480), (2304, 1152),
                                  (37888, 256), (38144, 640), (1024, 28672), (8192, 512), (8192, 896)])
 @pytest.mark.parametrize("m,groupsize", [(1, 128), (5, -1), (8, 128), (9, -1), (16, 128)])
