@@ -99,7 +99,13 @@ struct StreamCtx {
 constexpr int MAX_GRID = 256;
 
 std::mutex g_mu;
-std::atomic<uint64_t> g_launches{0};   // GEMMs and peer barriers this process has begun to launch, on any stream
+// Launches of this process's GEMMs and peer barriers, on any stream, counted before and after each; and records of the
+// host-buffer chain (w4a16_host_chain.h)
+std::atomic<uint64_t> g_count{0};
+struct CountLaunch {
+  CountLaunch() { g_count.fetch_add(1); }
+  ~CountLaunch() { g_count.fetch_add(1); }
+};
 std::map<std::pair<int, cudaStream_t>, StreamCtx> g_ctx;
 int g_sm_count[64] = {0};
 
@@ -965,8 +971,15 @@ int launch_decode_g(const Problem &pr) {
   return g ? launch_single<DecodeKernel<true, OUT_PLAIN>>(pr) : launch_single<DecodeKernel<false, OUT_PLAIN>>(pr);
 }
 
+int dispatch_tc(const Problem &pr);
+
+// The GEMM of every entry point; w4a16_plan, which launches nothing, calls dispatch_tc itself.
+int run_tc(const Problem &pr) {
+  const CountLaunch counted;
+  return dispatch_tc(pr);
+}
+
 int dispatch_tc(const Problem &pr) {
-  if (!pr.plan) g_launches.fetch_add(1);
   // batch tile = UMMA N; the k per stage is as deep as the activation tile allows (fewer, larger TMAs)
   const bool k256 = (pr.k % 256) == 0, k128 = (pr.k % 128) == 0;
   // Up to 8 rows: mma.sync on half-SM CTAs (us per launch in a chain at m = 1, before -> after: 512 x 1024 5.0 -> 2.2,
@@ -1152,7 +1165,7 @@ int gemm_entry(bool simt, const void *A, const void *B, void *C, const void *s, 
   if (!device_is_current(dev)) return W4A16_ERR_ARG;
   Problem pr{A, B, s, C, prob_m, prob_n, prob_k, groupsize, dev, sms, stream};
   pr.C2 = C2;
-  return simt ? launch_simt(pr) : dispatch_tc(pr);
+  return simt ? launch_simt(pr) : run_tc(pr);
 }
 
 }  // namespace
@@ -1281,10 +1294,12 @@ extern "C" int w4a16_marlin_gemm_host(const void *A_host, const void *B, void *C
 
   bool direct = false;
   w4a16::CopyIn how = w4a16::COPY_FIRST;
+  uint64_t seen = 0;
   if (g_host_direct != 0 && a_bytes <= HOST_COPY_MAX && c_bytes <= HOST_COPY_MAX) {
     std::lock_guard<std::mutex> lock(g_mu);
     direct = g_host_direct == 1 || g_host_chain.same_stream(dev, stream);
-    how = g_host_chain.order(dev, stream, g_launches.load(), bufs);
+    seen = g_count.load();
+    how = g_host_chain.order(dev, stream, seen, bufs);
   }
   void *dA = nullptr, *dC = nullptr;
   if (direct) {
@@ -1304,10 +1319,11 @@ extern "C" int w4a16_marlin_gemm_host(const void *A_host, const void *B, void *C
   if (rc == W4A16_OK && !direct && !cuda_ok(cudaMemcpyAsync(C_host, C_stage, c_bytes, cudaMemcpyDeviceToHost, st), "cudaMemcpyAsync(C)"))
     rc = W4A16_ERR_CUDA;
   std::lock_guard<std::mutex> lock(g_mu);
-  if (rc == W4A16_OK)
-    g_host_chain.record(dev, stream, direct ? g_launches.load() : 0, direct ? how : w4a16::COPY_FIRST, bufs);
+  const uint64_t now = g_count.fetch_add(1);
+  if (rc == W4A16_OK && direct)
+    g_host_chain.record(dev, stream, seen, now, how, bufs);
   else
-    g_host_chain.forget();
+    g_host_chain.forget(dev, stream);
   return rc;
 }
 
@@ -1384,7 +1400,7 @@ extern "C" int w4a16_marlin_gemm_builtin_scratch(const void *A, const void *B, v
     pr.fixed_status = g_builtin[dev].status;
     pr.fixed_slots = BUILTIN_SLOTS;
   }
-  return dispatch_tc(pr);
+  return run_tc(pr);
 }
 
 // Self-test of the bounded waits: the GEMM is set up so that the CTA finishing tile 0 expects a partial tile
@@ -1415,7 +1431,7 @@ extern "C" int w4a16_selftest_unanswered_wait(const void *A, const void *B, void
     pr.fixed_status = g_builtin[dev].status;
     pr.fixed_slots = BUILTIN_SLOTS;
   }
-  return dispatch_tc(pr);
+  return run_tc(pr);
 }
 
 extern "C" int w4a16_workspace_ints(int prob_n, int max_par) {
@@ -1542,7 +1558,7 @@ extern "C" int w4a16_marlin_gemm_gather(const void *A, const void *B, const void
     }
     pr.C_extra = static_cast<void *const *>(tab);
   }
-  return dispatch_tc(pr);
+  return run_tc(pr);
 }
 
 extern "C" int w4a16_peer_alloc(size_t bytes, void **dptr, void *handle64) {
@@ -1625,7 +1641,7 @@ extern "C" int w4a16_peer_barrier(void *const *flags, int world, int rank, int d
   }
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   int *status = nullptr;
-  g_launches.fetch_add(1);
+  const CountLaunch counted;
   {
     std::lock_guard<std::mutex> lock(g_mu);
     StreamCtx *ctx = get_ctx(dev, st, 0);

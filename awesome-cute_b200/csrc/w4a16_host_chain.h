@@ -6,6 +6,11 @@
 // before it has waited itself, and the copy-in of COPY_EARLY and COPY_LATE does the same: what such a chain has in front of it
 // when it starts goes back, kernel by kernel, to the last one that waited FIRST, and all calls since then may be unfinished.
 // Those are the open calls.
+//
+// Other threads may launch meanwhile, on this stream or others, and only what is known to be in front of a copy-in can be taken
+// for the open calls.  So the process counts its launches, once before and once after each, and the records of the chain: a
+// call that finds the counter where the last record has left it, and that record's call itself saw nothing but its own two
+// counts between its decision and its record, has nothing else between itself and that call.
 #pragma once
 #include <stddef.h>
 #include <stdint.h>
@@ -30,9 +35,9 @@ class HostChain {
   // The last call of this kind was on this stream.
   bool same_stream(int dev, const void *stream) const { return any_ && dev_ == dev && stream_ == stream; }
 
-  // launches: the process's launch counter now
-  CopyIn order(int dev, const void *stream, uint64_t launches, const HostBuffers &b) const {
-    if (!same_stream(dev, stream) || launches_ == 0 || launches_ != launches || open_.size() >= MAX_OPEN) return COPY_FIRST;
+  // count: the process's counter now
+  CopyIn order(int dev, const void *stream, uint64_t count, const HostBuffers &b) const {
+    if (!same_stream(dev, stream) || count_ == 0 || count_ != count || open_.size() >= MAX_OPEN) return COPY_FIRST;
     for (const HostBuffers &o : open_)   // what the copy-in reads and writes
       if (overlap(b.a_host, b.a_bytes, o.c_host, o.c_bytes) || overlap(b.a_stage, b.a_bytes, o.c_stage, o.c_bytes) ||
           overlap(b.a_stage, b.a_bytes, o.a_stage, o.a_bytes))
@@ -40,15 +45,16 @@ class HostChain {
     return COPY_EARLY;
   }
 
-  // After the call.  launches: the counter after it, or 0 when its copies went through the copy engines.
-  void record(int dev, const void *stream, uint64_t launches, CopyIn how, const HostBuffers &b) {
-    any_ = true, dev_ = dev, stream_ = stream, launches_ = launches;
+  // After the call.  seen: the counter at its decision; now: the counter before this record's own count.
+  void record(int dev, const void *stream, uint64_t seen, uint64_t now, CopyIn how, const HostBuffers &b) {
+    any_ = true, dev_ = dev, stream_ = stream;
+    count_ = now == seen + 2 ? now + 1 : 0;
     if (how == COPY_FIRST) open_.clear();
     open_.push_back(b);
   }
 
-  // After a call that failed half-way: what it has launched is not known.
-  void forget() { launches_ = 0; }
+  // After a call that went through the copy engines, or failed half-way: the next copy-in waits first.
+  void forget(int dev, const void *stream) { any_ = true, dev_ = dev, stream_ = stream, count_ = 0; }
 
  private:
   static bool overlap(const void *a, size_t na, const void *b, size_t nb) {
@@ -59,7 +65,7 @@ class HostChain {
   bool any_ = false;
   int dev_ = 0;
   const void *stream_ = nullptr;
-  uint64_t launches_ = 0;
+  uint64_t count_ = 0;
   std::vector<HostBuffers> open_;
 };
 

@@ -7,11 +7,11 @@ using w4a16::HostChain;
 extern "C" {
 void *chain_new() { return new HostChain; }
 void chain_delete(void *c) { delete static_cast<HostChain *>(c); }
-int chain_order(void *c, int dev, const void *stream, uint64_t launches, const HostBuffers *b) {
-  return static_cast<HostChain *>(c)->order(dev, stream, launches, *b);
+int chain_order(void *c, int dev, const void *stream, uint64_t count, const HostBuffers *b) {
+  return static_cast<HostChain *>(c)->order(dev, stream, count, *b);
 }
-void chain_record(void *c, int dev, const void *stream, uint64_t launches, int how, const HostBuffers *b) {
-  static_cast<HostChain *>(c)->record(dev, stream, launches, static_cast<w4a16::CopyIn>(how), *b);
+void chain_record(void *c, int dev, const void *stream, uint64_t seen, uint64_t now, int how, const HostBuffers *b) {
+  static_cast<HostChain *>(c)->record(dev, stream, seen, now, static_cast<w4a16::CopyIn>(how), *b);
 }
-void chain_forget(void *c) { static_cast<HostChain *>(c)->forget(); }
+void chain_forget(void *c, int dev, const void *stream) { static_cast<HostChain *>(c)->forget(dev, stream); }
 }

@@ -2,7 +2,8 @@
 
 The model knows of every kernel when it may start and when it lets its successor start, and so which earlier kernels may still
 be running when it touches its buffers.  Random sequences of host-buffer calls, GEMMs on device buffers and work of other
-origin, over a handful of buffers, must never touch what a kernel that may still be running reads or writes."""
+origin, over a handful of buffers and from one or several threads, must never touch what a kernel that may still be running
+reads or writes."""
 import ctypes
 import os
 import random
@@ -28,8 +29,8 @@ def library():
     lib.chain_new.restype = vp
     lib.chain_delete.argtypes = [vp]
     lib.chain_order.argtypes = [vp, ci, vp, u64, bp]
-    lib.chain_record.argtypes = [vp, ci, vp, u64, ci, bp]
-    lib.chain_forget.argtypes = [vp]
+    lib.chain_record.argtypes = [vp, ci, vp, u64, u64, ci, bp]
+    lib.chain_forget.argtypes = [vp, ci, vp]
     return lib
 
 
@@ -41,33 +42,43 @@ def clash(a, b):
     return any(x < y + m and y < x + n for x, n in a for y, m in b)
 
 
+class Call:
+    """A call of one thread: when it began and, once it has returned, when it did."""
+
+    def __init__(self, began=0):
+        self.began, self.returned = began, None
+
+
 class Stream:
-    """One stream.  A kernel: the earlier kernels that are over when it starts, and when it lets its successor start."""
+    """One stream.  A kernel: the earlier kernels that are over when it starts, and when it lets its successor start.  Only
+    what calls that had returned before a call began have launched is in order with that call."""
 
     def __init__(self, first_signals="after its wait"):
-        self.kernels = []           # (reads, writes, over at its start, signal)
+        self.kernels = []           # (reads, writes, over at its start, signal, call)
         self.first_signals = first_signals
+        self.call = Call()          # the call that launches
 
     def launch(self, reads, writes, signal, access="after its wait", ordinary=False):
         i = len(self.kernels)
         everything = set(range(i))
         over = everything
         if i and not ordinary:      # programmatic launch: starts when the one before lets it
-            _, _, before, sig = self.kernels[-1]
+            _, _, before, sig, _ = self.kernels[-1]
             over = before if sig == "at its start" else set(range(i - 1)) if sig == "after its wait" else everything
         # (a kernel that has waited has waited for everything before it: none ends before it has)
         for j in everything - (over if access == "at its start" else everything):
-            r, w = self.kernels[j][:2]
-            if clash(reads, w) or clash(writes, r) or clash(writes, w):
+            r, w, _, _, call = self.kernels[j]
+            ordered = call is self.call or call.returned is not None and call.returned <= self.call.began
+            if ordered and (clash(reads, w) or clash(writes, r) or clash(writes, w)):
                 raise Race("kernel %d touches what kernel %d, possibly unfinished, uses" % (i, j))
-        self.kernels.append((reads, writes, over, signal))
+        self.kernels.append((reads, writes, over, signal, self.call))
 
-    def host_call(self, how, b):
-        a_host, a_stage = (b.a_host, b.a_bytes), (b.a_stage, b.a_bytes)
-        c_stage, c_host = (b.c_stage, b.c_bytes), (b.c_host, b.c_bytes)
-        self.launch([a_host], [a_stage], self.first_signals if how == FIRST else "at its start",
+    def copy_in(self, how, b):
+        self.launch([(b.a_host, b.a_bytes)], [(b.a_stage, b.a_bytes)], self.first_signals if how == FIRST else "at its start",
                     "at its start" if how == EARLY else "after its wait")
-        self.launch([a_stage], [c_stage, c_host], "at its start")
+
+    def gemm(self, b):
+        self.launch([(b.a_stage, b.a_bytes)], [(b.c_stage, b.c_bytes), (b.c_host, b.c_bytes)], "at its start")
 
     def mul(self, a, c):
         self.launch([a], [c], "at its start")
@@ -76,23 +87,61 @@ class Stream:
         self.launch([a], [c], "at its end", ordinary=True)
 
 
-class Caller:
-    """The library's side: the launch counter and the chain."""
+class Library:
+    """The library's side: the process's counter and the chain.  host() and mul() are one call each, step by step."""
 
-    def __init__(self, lib, stream):
-        self.lib, self.chain, self.stream, self.launches = lib, lib.chain_new(), stream, 0
+    def __init__(self, lib, streams):
+        self.lib, self.chain, self.streams, self.count = lib, lib.chain_new(), streams, 0
+        self.clock = 0
         self.taken = []
 
-    def host(self, b):
-        how = self.lib.chain_order(self.chain, 0, 1, self.launches, b)
-        self.stream.host_call(how, b)
-        self.launches += 1
-        self.lib.chain_record(self.chain, 0, 1, self.launches, how, b)
-        self.taken.append(how)
+    def __del__(self):
+        self.lib.chain_delete(self.chain)
 
-    def mul(self, a, c):
-        self.stream.mul(a, c)
-        self.launches += 1
+    def tick(self):
+        self.clock += 1
+        return self.clock
+
+    def on(self, stream, call):
+        self.streams[stream].call = call
+        return self.streams[stream]
+
+    def host(self, stream, b):
+        call = Call(self.tick())
+        seen = self.count
+        how = self.lib.chain_order(self.chain, 0, stream + 1, seen, b)
+        self.taken.append(how)
+        yield
+        self.on(stream, call).copy_in(how, b)
+        yield
+        self.count += 1
+        yield
+        self.on(stream, call).gemm(b)
+        yield
+        self.count += 1
+        yield
+        self.lib.chain_record(self.chain, 0, stream + 1, seen, self.count, how, b)
+        self.count += 1
+        call.returned = self.tick()
+
+    def mul(self, stream, a, c):
+        call = Call(self.tick())
+        self.count += 1
+        yield
+        self.on(stream, call).mul(a, c)
+        yield
+        self.count += 1
+        call.returned = self.tick()
+
+    def other(self, stream, a, c):
+        call = Call(self.tick())
+        self.on(stream, call).other(a, c)
+        call.returned = self.tick()
+        yield
+
+    def run(self, call):
+        for _ in call:
+            pass
 
 
 def layer(i, o, size=64):
@@ -100,28 +149,38 @@ def layer(i, o, size=64):
     return Buffers(0x1000 * (1 + i), 0x100000 + 0x1000 * i, 0x200000 + 0x1000 * o, 0x1000 * (1 + o), size, size)
 
 
-def sequence(lib, seed, **kw):
+def sequence(lib, seed, threads=1, streams=1, **kw):
+    """Every thread makes its calls one after the other; the threads' steps are interleaved at random."""
     rng = random.Random(seed)
     host = [0x1000 * i for i in range(1, 9)]
     dev = [0x100000 + 0x1000 * i for i in range(1, 9)]
-    caller = Caller(lib, Stream(**kw))
     few = rng.choice([3, 8])
-    for _ in range(30):
-        kind = rng.choice(["host"] * 6 + ["mul", "other"])
-        pick = lambda pool: rng.choice(pool[:few]) + rng.choice([0, 0, 0, 32])
-        if kind == "host":
-            caller.host(Buffers(pick(host), pick(dev), pick(dev), pick(host), 64, 64))
-        elif kind == "mul":
-            caller.mul((pick(dev), 64), (pick(dev), 64))
-        else:
-            caller.stream.other((pick(host + dev), 64), (pick(host + dev), 64))
-    lib.chain_delete(caller.chain)
+    pick = lambda pool: (rng.choice(pool[:few]) + rng.choice([0, 0, 0, 32]), 64)
+    library = Library(lib, [Stream(**kw) for _ in range(streams)])
+
+    def thread():
+        for _ in range(30):
+            kind, stream = rng.choice(["host"] * 6 + ["mul", "other"]), rng.randrange(streams)
+            if kind == "host":
+                yield from library.host(stream, Buffers(pick(host)[0], pick(dev)[0], pick(dev)[0], pick(host)[0], 64, 64))
+            else:
+                pool = dev if kind == "mul" else host + dev
+                yield from getattr(library, kind)(stream, pick(pool), pick(pool))
+
+    running = [thread() for _ in range(threads)]
+    while running:
+        t = rng.choice(running)
+        for _ in range(rng.choice([1, 1, 3, 20])):
+            if next(t, t) is t:
+                running.remove(t)
+                break
 
 
-def test_no_call_touches_what_may_be_in_use():
+@pytest.mark.parametrize("threads,streams", [(1, 1), (1, 2), (2, 1), (2, 2), (3, 2)])
+def test_no_call_touches_what_may_be_in_use(threads, streams):
     lib = library()
-    for seed in range(3000):
-        sequence(lib, seed)
+    for seed in range(1500):
+        sequence(lib, seed, threads, streams)
 
 
 def test_the_model_sees_a_copy_in_that_signals_before_it_waits():
@@ -135,19 +194,35 @@ def test_the_model_sees_a_copy_in_that_signals_before_it_waits():
 
 def test_what_each_kind_of_sequence_costs():
     lib = library()
-    caller = Caller(lib, Stream())              # layers that share nothing: one call in eight waits first
-    for i in range(27):
-        caller.host(layer(2 * i, 2 * i + 1))
-    assert caller.taken == ([FIRST] + [EARLY] * 7) * 3 + [FIRST, EARLY, EARLY]
-    caller = Caller(lib, Stream())              # each reads what the one before has written: the GEMM still prefetches
+    calls = Library(lib, [Stream()])            # layers that share nothing: one call in eight waits first
+    for i in range(19):
+        calls.run(calls.host(0, layer(2 * i, 2 * i + 1)))
+    assert calls.taken == ([FIRST] + [EARLY] * 7) * 2 + [FIRST, EARLY, EARLY]
+    calls = Library(lib, [Stream()])            # each reads what the one before has written: the GEMM still prefetches
     for i in range(6):
-        caller.host(layer(i, i + 1))
-    assert caller.taken == [FIRST] + [LATE] * 5
-    caller.mul((1, 1), (3, 1))                  # a GEMM whose buffers the chain does not know
-    caller.host(layer(20, 21))
-    assert caller.taken[-1] == FIRST
-    caller.host(layer(22, 23))
-    assert caller.taken[-1] == EARLY
-    lib.chain_forget(caller.chain)
-    caller.host(layer(24, 25))
-    assert caller.taken[-1] == FIRST
+        calls.run(calls.host(0, layer(i, i + 1)))
+    assert calls.taken == [FIRST] + [LATE] * 5
+    calls.run(calls.mul(0, (1, 1), (3, 1)))     # a GEMM whose buffers the chain does not know
+    for i, want in ((20, FIRST), (22, EARLY)):
+        calls.run(calls.host(0, layer(i, i + 1)))
+        assert calls.taken[-1] == want
+    lib.chain_forget(calls.chain, 0, 1)
+    calls.run(calls.host(0, layer(24, 25)))
+    assert calls.taken[-1] == FIRST
+
+
+def test_a_launch_of_another_thread_in_the_middle_of_a_call():
+    """A GEMM that another thread enqueues between a call's own launches and its record is not taken for the call's own."""
+    lib = library()
+    calls = Library(lib, [Stream()])
+    calls.run(calls.host(0, layer(0, 1)))
+    for steps in range(1, 6):
+        for i in (2, 6):                        # (the first one alone, so that the second finds the chain whole)
+            call = calls.host(0, layer(10 * steps + i, 10 * steps + i + 1))
+            if i == 6:
+                for _ in range(steps):
+                    next(call)
+                calls.run(calls.mul(0, (0x100000 + 0x1000 * 99, 64), (3, 1)))
+            calls.run(call)
+        calls.run(calls.host(0, Buffers(0x99000, 0x100000 + 0x1000 * 99, 0x5000000, 0x98000, 64, 64)))
+        assert calls.taken[-1] == FIRST, steps
