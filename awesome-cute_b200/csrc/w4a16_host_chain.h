@@ -21,7 +21,7 @@ namespace w4a16 {
 
 enum CopyIn {
   COPY_FIRST = 0,   // waits, then lets the GEMM behind it start: everything before is over for all that follows
-  COPY_LATE = 1,    // lets the GEMM start (it prefetches its weights), waits, copies: shares a buffer with an open call
+  COPY_LATE = 1,    // lets the GEMM start (it prefetches its weights), waits, copies: shares a buffer with the last call only
   COPY_EARLY = 2,   // copies beside the open calls' GEMMs and waits at its end: shares none
 };
 
@@ -38,10 +38,15 @@ class HostChain {
   // count: the process's counter now
   CopyIn order(int dev, const void *stream, uint64_t count, const HostBuffers &b) const {
     if (!same_stream(dev, stream) || count_ == 0 || count_ != count || open_.size() >= MAX_OPEN) return COPY_FIRST;
-    for (const HostBuffers &o : open_)   // what the copy-in reads and writes
+    // What the copy-in reads and writes.  A buffer shared with the call right before is waited for anyway; one shared with an
+    // older call (a buffer that comes back) closes the list instead of making every later call wait for its predecessor: four
+    // layers with buffers of their own, called over and over, wait once a pass.
+    for (size_t i = 0; i < open_.size(); ++i) {
+      const HostBuffers &o = open_[i];
       if (overlap(b.a_host, b.a_bytes, o.c_host, o.c_bytes) || overlap(b.a_stage, b.a_bytes, o.c_stage, o.c_bytes) ||
           overlap(b.a_stage, b.a_bytes, o.a_stage, o.a_bytes))
-        return COPY_LATE;
+        return i + 1 < open_.size() ? COPY_FIRST : COPY_LATE;
+    }
     return COPY_EARLY;
   }
 

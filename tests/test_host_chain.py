@@ -202,6 +202,12 @@ def test_what_each_kind_of_sequence_costs():
     for i in range(6):
         calls.run(calls.host(0, layer(i, i + 1)))
     assert calls.taken == [FIRST] + [LATE] * 5
+    calls.run(calls.host(0, layer(4, 9)))       # a fan-out: the second reader of a result
+    assert calls.taken[-1] == FIRST
+    calls = Library(lib, [Stream()])            # four layers over and over, each with buffers of its own
+    for i in range(12):
+        calls.run(calls.host(0, layer(2 * (i % 4), 2 * (i % 4) + 1)))
+    assert calls.taken == [FIRST, EARLY, EARLY, EARLY] * 3
     calls.run(calls.mul(0, (1, 1), (3, 1)))     # a GEMM whose buffers the chain does not know
     for i, want in ((20, FIRST), (22, EARLY)):
         calls.run(calls.host(0, layer(i, i + 1)))
