@@ -1259,6 +1259,15 @@ void *device_view_of_host(const void *host, size_t bytes) {
 
 w4a16::HostChain g_host_chain;   // guarded by g_mu
 
+bool place_of(int dev, cudaStream_t st, w4a16::Place &p) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  p = w4a16::Place{dev, st, 0, 0};
+  if (!cuda_ok(cudaStreamGetCaptureInfo(st, &status, &p.capture), "cudaStreamGetCaptureInfo")) return false;
+  if (status != cudaStreamCaptureStatusNone) return true;   // (a capture does not allow the question below)
+  p.capture = 0;
+  return cuda_ok(cudaStreamGetId(st, &p.id), "cudaStreamGetId");
+}
+
 int launch_copy_in(const void *src, void *dst, size_t bytes, cudaStream_t st, w4a16::CopyIn how) {
   cudaLaunchConfig_t cfg = {};
   // few SMs: one block per 64 KB, at most 16 (PCIe, not the SMs, bounds it), so that the GEMM's CTAs find theirs free
@@ -1295,11 +1304,13 @@ extern "C" int w4a16_marlin_gemm_host(const void *A_host, const void *B, void *C
   bool direct = false;
   w4a16::CopyIn how = w4a16::COPY_FIRST;
   uint64_t seen = 0;
+  w4a16::Place place;
+  if (!place_of(dev, st, place)) return W4A16_ERR_CUDA;
   if (g_host_direct != 0 && a_bytes <= HOST_COPY_MAX && c_bytes <= HOST_COPY_MAX) {
     std::lock_guard<std::mutex> lock(g_mu);
-    direct = g_host_direct == 1 || g_host_chain.same_stream(dev, stream);
+    direct = g_host_direct == 1 || g_host_chain.same_stream(place);
     seen = g_count.load();
-    how = g_host_chain.order(dev, stream, seen, bufs);
+    how = g_host_chain.order(place, seen, bufs);
   }
   void *dA = nullptr, *dC = nullptr;
   if (direct) {
@@ -1321,9 +1332,9 @@ extern "C" int w4a16_marlin_gemm_host(const void *A_host, const void *B, void *C
   std::lock_guard<std::mutex> lock(g_mu);
   const uint64_t now = g_count.fetch_add(1);
   if (rc == W4A16_OK && direct)
-    g_host_chain.record(dev, stream, seen, now, how, bufs);
+    g_host_chain.record(place, seen, now, how, bufs);
   else
-    g_host_chain.forget(dev, stream);
+    g_host_chain.forget(place);
   return rc;
 }
 

@@ -30,14 +30,24 @@ struct HostBuffers {
   size_t a_bytes, c_bytes;
 };
 
+// Where a call's work goes.  capture: 0, or the id of the capture that the stream is in: captured work is not in front of what
+// the stream runs next, nor the other way round.  id: outside of a capture the stream's id, which no other stream of the process
+// ever has (a handle may come back, and that of the per-thread default stream stands for one stream per thread).
+struct Place {
+  int dev;
+  const void *stream;
+  unsigned long long id, capture;
+  bool operator==(const Place &o) const { return dev == o.dev && stream == o.stream && id == o.id && capture == o.capture; }
+};
+
 class HostChain {
  public:
   // The last call of this kind was on this stream.
-  bool same_stream(int dev, const void *stream) const { return any_ && dev_ == dev && stream_ == stream; }
+  bool same_stream(const Place &p) const { return any_ && place_.dev == p.dev && place_.stream == p.stream; }
 
   // count: the process's counter now
-  CopyIn order(int dev, const void *stream, uint64_t count, const HostBuffers &b) const {
-    if (!same_stream(dev, stream) || count_ == 0 || count_ != count || open_.size() >= MAX_OPEN) return COPY_FIRST;
+  CopyIn order(const Place &p, uint64_t count, const HostBuffers &b) const {
+    if (!any_ || !(place_ == p) || count_ == 0 || count_ != count || open_.size() >= MAX_OPEN) return COPY_FIRST;
     // What the copy-in reads and writes.  A buffer shared with the call right before is waited for anyway; one shared with an
     // older call (a buffer that comes back) closes the list instead of making every later call wait for its predecessor: four
     // layers with buffers of their own, called over and over, wait once a pass.
@@ -51,15 +61,15 @@ class HostChain {
   }
 
   // After the call.  seen: the counter at its decision; now: the counter before this record's own count.
-  void record(int dev, const void *stream, uint64_t seen, uint64_t now, CopyIn how, const HostBuffers &b) {
-    any_ = true, dev_ = dev, stream_ = stream;
+  void record(const Place &p, uint64_t seen, uint64_t now, CopyIn how, const HostBuffers &b) {
+    any_ = true, place_ = p;
     count_ = now == seen + 2 ? now + 1 : 0;
     if (how == COPY_FIRST) open_.clear();
     open_.push_back(b);
   }
 
   // After a call that went through the copy engines, or failed half-way: the next copy-in waits first.
-  void forget(int dev, const void *stream) { any_ = true, dev_ = dev, stream_ = stream, count_ = 0; }
+  void forget(const Place &p) { any_ = true, place_ = p, count_ = 0; }
 
  private:
   static bool overlap(const void *a, size_t na, const void *b, size_t nb) {
@@ -68,8 +78,7 @@ class HostChain {
   }
   static constexpr size_t MAX_OPEN = 8;
   bool any_ = false;
-  int dev_ = 0;
-  const void *stream_ = nullptr;
+  Place place_{};
   uint64_t count_ = 0;
   std::vector<HostBuffers> open_;
 };

@@ -3,15 +3,16 @@
 
 using w4a16::HostBuffers;
 using w4a16::HostChain;
+using w4a16::Place;
 
 extern "C" {
 void *chain_new() { return new HostChain; }
 void chain_delete(void *c) { delete static_cast<HostChain *>(c); }
-int chain_order(void *c, int dev, const void *stream, uint64_t count, const HostBuffers *b) {
-  return static_cast<HostChain *>(c)->order(dev, stream, count, *b);
+int chain_order(void *c, const Place *p, uint64_t count, const HostBuffers *b) {
+  return static_cast<HostChain *>(c)->order(*p, count, *b);
 }
-void chain_record(void *c, int dev, const void *stream, uint64_t seen, uint64_t now, int how, const HostBuffers *b) {
-  static_cast<HostChain *>(c)->record(dev, stream, seen, now, static_cast<w4a16::CopyIn>(how), *b);
+void chain_record(void *c, const Place *p, uint64_t seen, uint64_t now, int how, const HostBuffers *b) {
+  static_cast<HostChain *>(c)->record(*p, seen, now, static_cast<w4a16::CopyIn>(how), *b);
 }
-void chain_forget(void *c, int dev, const void *stream) { static_cast<HostChain *>(c)->forget(dev, stream); }
+void chain_forget(void *c, const Place *p) { static_cast<HostChain *>(c)->forget(*p); }
 }

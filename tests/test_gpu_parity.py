@@ -559,6 +559,40 @@ def test_host_calls_that_share_buffers(m, d):
         assert torch.equal(h[5].to(DEV), mul(h[4], 5))
 
 
+@pytest.mark.parametrize("m", [4, 40])
+def test_captured_host_calls_between_eager_ones(m):
+    """Calls with host buffers in a CUDA graph, replayed between eager ones on the same stream and the same staging buffers."""
+    d = 512
+    gen = torch.Generator(device=DEV).manual_seed(m)
+    Bs = [torch.randint(-2 ** 31, 2 ** 31, (d // 16, 2 * d), generator=gen, device=DEV, dtype=torch.int) for _ in range(4)]
+    s = torch.full((d // 128, d), 0.2 * d ** -0.5, device=DEV, dtype=torch.half)
+    ws = torch.zeros(d // 128 * 16, dtype=torch.int, device=DEV)
+    sa, sc = [[torch.zeros((m, d), dtype=torch.half, device=DEV) for _ in range(2)] for _ in range(2)]
+    h = [torch.zeros((m, d), dtype=torch.half).pin_memory() for _ in range(5)]
+    stream = torch.cuda.Stream()
+    ops = [pkg.HostGemm(h[i], Bs[i], h[i + 1], s, ws, sa[i % 2], sc[i % 2], stream=stream) for i in range(4)]
+    for op in ops:
+        op()
+    stream.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        ops[1]()
+        ops[2]()
+    for _ in range(4):
+        h[0].copy_(torch.randn((m, d), generator=gen, device=DEV).half())
+        torch.cuda.synchronize()
+        with torch.cuda.stream(stream):
+            ops[0]()
+            graph.replay()
+            ops[3]()
+        stream.synchronize()
+        for i in range(4):
+            c = torch.zeros((m, d), dtype=torch.half, device=DEV)
+            pkg.mul(h[i].to(DEV), Bs[i], c, s, ws)
+            assert torch.equal(c.cpu(), h[i + 1]), i
+    pkg.device_status(0)
+
+
 @pytest.mark.parametrize("n,k", [(128, 128), (256, 512), (128, 11008), (4096, 4096), (8192, 8192), (1280, 4480), (2304, 1152),
                                  (37888, 256), (38144, 640), (1024, 28672), (8192, 512), (8192, 896)])
 @pytest.mark.parametrize("m,groupsize", [(1, 128), (5, -1), (8, 128), (9, -1), (16, 128)])

@@ -21,16 +21,20 @@ class Buffers(ctypes.Structure):
         (n, ctypes.c_size_t) for n in ("a_bytes", "c_bytes")]
 
 
+class Place(ctypes.Structure):
+    _fields_ = [("dev", ctypes.c_int), ("stream", ctypes.c_void_p), ("id", ctypes.c_ulonglong), ("capture", ctypes.c_ulonglong)]
+
+
 def library():
     if not os.path.exists(LIB):
         entry._make(os.path.dirname(LIB))
     lib = ctypes.CDLL(LIB)
-    vp, ci, u64, bp = ctypes.c_void_p, ctypes.c_int, ctypes.c_uint64, ctypes.POINTER(Buffers)
+    vp, ci, u64, bp, pp = ctypes.c_void_p, ctypes.c_int, ctypes.c_uint64, ctypes.POINTER(Buffers), ctypes.POINTER(Place)
     lib.chain_new.restype = vp
     lib.chain_delete.argtypes = [vp]
-    lib.chain_order.argtypes = [vp, ci, vp, u64, bp]
-    lib.chain_record.argtypes = [vp, ci, vp, u64, u64, ci, bp]
-    lib.chain_forget.argtypes = [vp, ci, vp]
+    lib.chain_order.argtypes = [vp, pp, u64, bp]
+    lib.chain_record.argtypes = [vp, pp, u64, u64, ci, bp]
+    lib.chain_forget.argtypes = [vp, pp]
     return lib
 
 
@@ -102,6 +106,9 @@ class Library:
         self.clock += 1
         return self.clock
 
+    def place(self, stream, capture=0):
+        return Place(0, stream + 1, 0 if capture else 1, capture)
+
     def on(self, stream, call):
         self.streams[stream].call = call
         return self.streams[stream]
@@ -109,7 +116,7 @@ class Library:
     def host(self, stream, b):
         call = Call(self.tick())
         seen = self.count
-        how = self.lib.chain_order(self.chain, 0, stream + 1, seen, b)
+        how = self.lib.chain_order(self.chain, self.place(stream), seen, b)
         self.taken.append(how)
         yield
         self.on(stream, call).copy_in(how, b)
@@ -120,7 +127,7 @@ class Library:
         yield
         self.count += 1
         yield
-        self.lib.chain_record(self.chain, 0, stream + 1, seen, self.count, how, b)
+        self.lib.chain_record(self.chain, self.place(stream), seen, self.count, how, b)
         self.count += 1
         call.returned = self.tick()
 
@@ -212,7 +219,7 @@ def test_what_each_kind_of_sequence_costs():
     for i, want in ((20, FIRST), (22, EARLY)):
         calls.run(calls.host(0, layer(i, i + 1)))
         assert calls.taken[-1] == want
-    lib.chain_forget(calls.chain, 0, 1)
+    lib.chain_forget(calls.chain, calls.place(0))
     calls.run(calls.host(0, layer(24, 25)))
     assert calls.taken[-1] == FIRST
 
@@ -232,3 +239,33 @@ def test_a_launch_of_another_thread_in_the_middle_of_a_call():
             calls.run(call)
         calls.run(calls.host(0, Buffers(0x99000, 0x100000 + 0x1000 * 99, 0x5000000, 0x98000, 64, 64)))
         assert calls.taken[-1] == FIRST, steps
+
+
+def test_captured_calls_are_not_in_front_of_eager_ones():
+    """A call that is captured runs at the graph's launch, not where the chain has seen it: what was open before the capture is
+    still open behind it, and the first call after it, as the first call inside it, waits first."""
+    lib = library()
+    calls = Library(lib, [Stream()])
+    calls.run(calls.host(0, layer(0, 1)))
+    order = lambda capture, b: lib.chain_order(calls.chain, calls.place(0, capture), calls.count, b)
+
+    def captured(capture, b):
+        seen, how = calls.count, order(capture, b)
+        calls.count += 2
+        lib.chain_record(calls.chain, calls.place(0, capture), seen, calls.count, how, b)
+        calls.count += 1
+        return how
+
+    assert order(0, layer(2, 3)) == EARLY
+    assert [captured(7, layer(i, i + 1)) for i in (4, 6, 7)] == [FIRST, EARLY, LATE]
+    assert captured(8, layer(20, 21)) == FIRST
+    assert order(0, layer(2, 3)) == FIRST
+    assert order(8, layer(2, 3)) == EARLY
+
+
+def test_a_handle_that_comes_back_is_another_stream():
+    lib = library()
+    calls = Library(lib, [Stream()])
+    calls.run(calls.host(0, layer(0, 1)))
+    for place, want in ((Place(0, 1, 1, 0), EARLY), (Place(0, 1, 2, 0), FIRST), (Place(1, 1, 1, 0), FIRST)):
+        assert lib.chain_order(calls.chain, place, calls.count, layer(2, 3)) == want
