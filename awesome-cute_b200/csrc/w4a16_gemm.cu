@@ -134,27 +134,35 @@ int l2_bytes(int dev) {
 // Must be called with g_mu held.  The scratch is sized by need: the first block covers every launch of up to 64 batch
 // rows on this device (one slot row per CTA row: SMs x 64 x 128 fp32, 4.8 MB on a 148-SM part), larger batch tiles
 // grow it (SMs x 192 x 128 fp32 = 14.5 MB at most).  Growing allocates, which CUDA refuses while a stream is being
-// captured: run a problem of the size once before capturing it.
-StreamCtx *get_ctx(int dev, cudaStream_t stream, size_t need_slots) {
+// captured: run a problem of the size once before capturing it.  A launch that needs no scratch itself (clusters) still
+// readies what the stream-K launches of its size need (ready_slots), unless its stream is being captured: a caller that has
+// run one layer may capture the others.
+StreamCtx *get_ctx(int dev, cudaStream_t stream, size_t need_slots, size_t ready_slots = 0) {
   StreamCtx &c = g_ctx[{dev, stream}];
   if (!c.status) {
     if (!cuda_ok(cudaMalloc(&c.status, sizeof(int)), "cudaMalloc(status)")) return nullptr;
     if (!cuda_ok(cudaMemset(c.status, 0, sizeof(int)), "cudaMemset(status)")) return nullptr;
   }
-  if (c.partial_slots < need_slots) {
-    const int nsm = sm_count(dev);
-    const size_t floor_slots = (size_t)(nsm > 0 ? nsm : MAX_GRID) * 64 * w4a16::TILE_N;
-    const size_t slots = std::max(need_slots, floor_slots);
-    uint32_t *blk = nullptr;
-    if (!cuda_ok(cudaMalloc(&blk, sizeof(uint32_t) * slots), "cudaMalloc(partials)")) return nullptr;
-    if (!cuda_ok(cudaMemset(blk, 0xff, sizeof(uint32_t) * slots), "cudaMemset(partials)")) {
-      cudaFree(blk);
-      return nullptr;
+  if (c.partial_slots >= need_slots) {
+    if (c.partial_slots >= ready_slots) return &c;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) {
+      cudaGetLastError();   // (the null stream while another stream is being captured)
+      return &c;
     }
-    if (c.partials) c.retired.emplace_back(c.partials, c.partial_slots);
-    c.partials = blk;
-    c.partial_slots = slots;
   }
+  const int nsm = sm_count(dev);
+  const size_t floor_slots = (size_t)(nsm > 0 ? nsm : MAX_GRID) * 64 * w4a16::TILE_N;
+  const size_t slots = std::max({need_slots, ready_slots, floor_slots});
+  uint32_t *blk = nullptr;
+  if (!cuda_ok(cudaMalloc(&blk, sizeof(uint32_t) * slots), "cudaMalloc(partials)")) return nullptr;
+  if (!cuda_ok(cudaMemset(blk, 0xff, sizeof(uint32_t) * slots), "cudaMemset(partials)")) {
+    cudaFree(blk);
+    return nullptr;
+  }
+  if (c.partials) c.retired.emplace_back(c.partials, c.partial_slots);
+  c.partials = blk;
+  c.partial_slots = slots;
   return &c;
 }
 
@@ -280,7 +288,7 @@ bool get_maps(const Problem &pr, int ks, int a_rows, bool grouped, bool tma_stor
 }
 
 // scratch + status word of this launch (library-owned per (device, stream), or the built-in array)
-bool get_scratch(const Problem &pr, size_t need_slots, w4a16::Params &p) {
+bool get_scratch(const Problem &pr, size_t need_slots, w4a16::Params &p, size_t ready_slots = 1) {
   if (pr.fixed_partials) {
     if (need_slots > pr.fixed_slots) {
       g_last_error = "problem needs " + std::to_string(need_slots) + " partial-tile slots, the built-in scratch holds " +
@@ -292,7 +300,7 @@ bool get_scratch(const Problem &pr, size_t need_slots, w4a16::Params &p) {
     return true;
   }
   std::lock_guard<std::mutex> lock(g_mu);
-  StreamCtx *ctx = get_ctx(pr.dev, pr.stream, need_slots);
+  StreamCtx *ctx = get_ctx(pr.dev, pr.stream, need_slots, ready_slots);
   if (!ctx) return false;
   p.partials = ctx->partials;
   p.status = ctx->status;
@@ -760,7 +768,7 @@ int launch_tc2_cluster(const Problem &pr) {
   Maps mp;
   if (!get_maps(pr, Cfg::KS, Cfg::HALF_ROWS, GROUPED, false, mp)) return W4A16_ERR_CUDA;
   if (!mp.a_box3d) return -2;
-  if (!get_scratch(pr, 0, p)) return W4A16_ERR_CUDA;   // the status word only
+  if (!get_scratch(pr, 0, p, (size_t)nsm * TM * w4a16::TILE_N)) return W4A16_ERR_CUDA;   // the status word only
   if (!cuda_ok(cudaLaunchKernelEx(&cfg, kern, mp.b, mp.a, mp.s, mp.c, p), "kernel launch (clusters of CTA pairs)")) return W4A16_ERR_CUDA;
   return W4A16_OK;
 }

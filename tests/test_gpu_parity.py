@@ -328,6 +328,37 @@ def test_dependent_chain_eager_and_graph_replay(m):
         verify("graph %d" % rep)
 
 
+@pytest.mark.parametrize("m,first,then", [(1, (512, 1024), (12288, 4096)), (16, (4096, 4096), (22016, 4096)),
+                                          (48, (1024, 2048), (22016, 1024)), (128, (4096, 4096), (12288, 4096))])
+def test_capture_after_one_layer_has_run(m, first, then):
+    """A call sets up what every launch of its batch size needs on the stream, also where it runs in clusters and needs no
+    scratch itself: a stream-K layer may be captured behind it."""
+    probs = []
+    for n, k in (first, then):
+        gen = torch.Generator(device=DEV).manual_seed(n + m)
+        probs.append((torch.randn((m, k), generator=gen, device=DEV).half(),
+                      torch.randint(-2 ** 31, 2 ** 31, (k // 16, 2 * n), generator=gen, device=DEV, dtype=torch.int),
+                      torch.zeros((m, n), dtype=torch.half, device=DEV),
+                      torch.full((k // 128, n), 0.01, dtype=torch.half, device=DEV),
+                      torch.zeros(n // 128 * 16, dtype=torch.int, device=DEV)))
+    stream = torch.cuda.Stream()
+    _lib = pkg._lib
+    assert _lib.lib.w4a16_release_stream(0, stream.cuda_stream) == _lib.OK    # (torch hands pooled streams out again)
+    torch.cuda.synchronize()
+    with torch.cuda.stream(stream):
+        pkg.mul(*probs[0])
+    stream.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        pkg.mul(*probs[1])
+    graph.replay()
+    torch.cuda.synchronize()
+    A, B, C, s, ws = probs[1]
+    again = torch.zeros_like(C)
+    pkg.mul(A, B, again, s, ws)
+    assert bool(C.any()) and torch.equal(C, again)
+
+
 def test_random_shapes_stress():
     """Many small random problems back to back on one stream (different tilings, split counts and scratch
     reuse patterns), each checked against the oracle."""
