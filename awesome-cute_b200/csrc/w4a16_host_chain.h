@@ -15,7 +15,7 @@
 #include <stddef.h>
 #include <stdint.h>
 
-#include <vector>
+#include <array>
 
 namespace w4a16 {
 
@@ -47,15 +47,15 @@ class HostChain {
 
   // count: the process's counter now
   CopyIn order(const Place &p, uint64_t count, const HostBuffers &b) const {
-    if (!any_ || !(place_ == p) || count_ == 0 || count_ != count || open_.size() >= MAX_OPEN) return COPY_FIRST;
+    if (!any_ || !(place_ == p) || count_ == 0 || count_ != count || n_open_ >= MAX_OPEN) return COPY_FIRST;
     // What the copy-in reads and writes.  A buffer shared with the call right before is waited for anyway; one shared with an
     // older call (a buffer that comes back) closes the list instead of making every later call wait for its predecessor: four
     // layers with buffers of their own, called over and over, wait once a pass.
-    for (size_t i = 0; i < open_.size(); ++i) {
+    for (size_t i = 0; i < n_open_; ++i) {
       const HostBuffers &o = open_[i];
       if (overlap(b.a_host, b.a_bytes, o.c_host, o.c_bytes) || overlap(b.a_stage, b.a_bytes, o.c_stage, o.c_bytes) ||
           overlap(b.a_stage, b.a_bytes, o.a_stage, o.a_bytes))
-        return i + 1 < open_.size() ? COPY_FIRST : COPY_LATE;
+        return i + 1 < n_open_ ? COPY_FIRST : COPY_LATE;
     }
     return COPY_EARLY;
   }
@@ -64,8 +64,11 @@ class HostChain {
   void record(const Place &p, uint64_t seen, uint64_t now, CopyIn how, const HostBuffers &b) {
     any_ = true, place_ = p;
     count_ = now == seen + 2 ? now + 1 : 0;
-    if (how == COPY_FIRST) open_.clear();
-    open_.push_back(b);
+    if (how == COPY_FIRST) n_open_ = 0;
+    if (n_open_ < MAX_OPEN)
+      open_[n_open_++] = b;
+    else
+      count_ = 0;   // (threads that decided at the same time)
   }
 
   // After a call that went through the copy engines, or failed half-way: the next copy-in waits first.
@@ -80,7 +83,8 @@ class HostChain {
   bool any_ = false;
   Place place_{};
   uint64_t count_ = 0;
-  std::vector<HostBuffers> open_;
+  std::array<HostBuffers, MAX_OPEN> open_{};
+  size_t n_open_ = 0;
 };
 
 }  // namespace w4a16
