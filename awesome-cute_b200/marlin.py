@@ -45,11 +45,14 @@ def mul(A, B, C, s, workspace, thread_k=-1, thread_n=-1, sms=-1, max_par=16, cut
     """
     # The compiled path serves every call that is right; what it leaves is checked here, for the error message.
     # (4096 x 4096 at m = 1: 8.5 us of host time per call through the code below, 3.7 us through it; Layer.forward 18.6 -> 6 us.)
-    if _entry is None and _calls.mul(A, B, C, s, workspace, thread_k, thread_n, sms, max_par):
+    err = _calls.mul(A, B, C, s, workspace, thread_k, thread_n, sms, max_par) if _calls and _entry is None else None
+    if err == 0:
         return
     prob_m, prob_k = A.shape[0], A.shape[1]
     prob_n = C.shape[1]
     groupsize = -1 if s.shape[0] == 1 else prob_k // s.shape[0]
+    if err is not None:
+        _check(err, prob_m, prob_n, prob_k, thread_k, thread_n, groupsize)
     if groupsize != -1 and groupsize * s.shape[0] != prob_k:
         raise RuntimeError("k=%d not compatible with %d groups." % (prob_k, s.shape[0]))
     need = prob_n // 128 * max_par      # w4a16_workspace_ints, computed here to keep the call path short
@@ -264,10 +267,13 @@ class Layer(nn.Module):
         self.register_buffer('workspace', torch.zeros(self.n // 128 * 16, dtype=torch.int), persistent=False)
 
     def forward(self, A):
-        b = self._buffers            # (attribute access would go through Module.__getattr__ for each of them)
-        C = _calls.forward(A, b['B'], b['s'], b['workspace'])
-        if C is not None:
-            return C
+        if _calls:
+            b = self._buffers        # (attribute access would go through Module.__getattr__ for each of them)
+            C = _calls.forward(A, b.get('B'), b.get('s'), b.get('workspace'))
+            if isinstance(C, int):
+                _check(C, A.numel() // self.k, self.n, self.k, -1, -1, -1 if self.groupsize == self.k else self.groupsize)
+            if C is not None:
+                return C
         C = torch.empty(A.shape[:-1] + (self.s.shape[1],), dtype=A.dtype, device=A.device)
         mul(A.view((-1, A.shape[-1])), self.B, C.view((-1, C.shape[-1])), self.s, self.workspace)
         return C
@@ -291,7 +297,9 @@ class Layer(nn.Module):
 def quantize_pack_device(weight_nk, scales, groupsize):
     """Layer.pack on the device: weight fp16 [n, k] (CUDA), scales fp16 [groups, n] (CUDA) -> (B int32 [k/16, 2n],
     s_packed fp16 [groups, n]) on the same device.  Bit-exact with quantize_pack()."""
-    out = _calls.quantize_pack(weight_nk, scales, groupsize)
+    out = _calls.quantize_pack(weight_nk, scales, groupsize) if _calls else None
+    if isinstance(out, int):
+        raise ValueError("w4a16_quantize_pack_device: code %d" % out)
     if out is not None:
         return out
     if not (weight_nk.is_cuda and scales.is_cuda):
