@@ -6,6 +6,7 @@ importing it raises.
 """
 import ctypes
 import os
+import warnings
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.environ.get("W4A16_LIB") or os.path.join(_HERE, "libw4a16.so")   # W4A16_LIB: debugging override
@@ -66,14 +67,15 @@ def _load_calls():
     try:
         from . import _torch_calls
     except ImportError as e:
-        raise ImportError("_torch_calls.so is not built, or for another torch (%s). Build it with "
-                          "`make -C awesome-cute_b200/csrc`." % e) from e
+        warnings.warn("_torch_calls.so is not built, or for another torch (%s): calls take the slower path through ctypes.  Build "
+                      "it with `make -C awesome-cute_b200/csrc`." % e, RuntimeWarning, stacklevel=2)
+        return None
     _torch_calls.bind(*(ctypes.cast(f, ctypes.c_void_p).value
                         for f in (lib.w4a16_marlin_gemm, lib.w4a16_quantize_pack_device)))
     return _torch_calls
 
 
-calls = _load_calls()   # the compiled path from torch tensors to the two entry points above
+calls = _load_calls()   # the compiled path from torch tensors to the two entry points above, or None
 
 
 class Plan(ctypes.Structure):

@@ -1,6 +1,9 @@
-"""The compiled call path (awesome-cute_b200/csrc/w4a16_torch.cpp) and what happens beside it: with an error of the
-library, on layers whose tensors are not plain buffers."""
+"""The compiled call path (awesome-cute_b200/csrc/w4a16_torch.cpp) and what happens beside it: without the module, with an
+error of the library, on layers whose tensors are not plain buffers."""
 import ctypes
+import os
+import subprocess
+import sys
 
 import pytest
 import torch
@@ -9,6 +12,48 @@ import __graft_entry__ as entry
 
 pkg = entry.load_package()
 from awesome_cute_b200 import _lib  # noqa: E402
+
+WITHOUT = r"""
+import sys, warnings
+sys.modules['awesome_cute_b200._torch_calls'] = None        # as if it were not built, or for another torch
+import torch
+import __graft_entry__ as entry
+with warnings.catch_warnings(record=True) as seen:
+    warnings.simplefilter('always')
+    pkg = entry.load_package()
+assert any('_torch_calls' in str(w.message) for w in seen), seen
+A, C = torch.zeros((16, 256), dtype=torch.half), torch.zeros((16, 256), dtype=torch.half)
+B, s = torch.zeros((16, 512), dtype=torch.int), torch.zeros((2, 256), dtype=torch.half)
+try:
+    pkg.mul(A, B, C, s, torch.zeros(32, dtype=torch.int))
+except RuntimeError as e:
+    assert 'no CPU implementation' in str(e), e
+layer = pkg.Layer(256, 256, 128)
+if torch.cuda.is_available():
+    layer = layer.cuda()
+    w, sc = torch.randn(256, 256).half().cuda(), torch.full((2, 256), 0.01).half().cuda()
+    layer.B, layer.s = pkg.quantize_pack_device(w, sc, 128)
+    x = torch.randn(3, 256).half().cuda()
+    y = torch.zeros(3, 256).half().cuda()
+    pkg.mul(x, layer.B, y, layer.s, layer.workspace)
+    assert torch.equal(layer(x), y) and bool(y.any())
+print('ok')
+"""
+
+
+def run_without():
+    r = subprocess.run([sys.executable, "-c", WITHOUT], cwd=entry.ROOT, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and r.stdout.strip() == "ok", r.stdout[-1000:] + r.stderr[-2000:]
+
+
+def test_the_package_works_without_the_module():
+    run_without()
+
+
+@pytest.mark.gpu
+def test_the_package_works_without_the_module_on_a_gpu():
+    run_without()
+
 
 def operands(m=4, n=256, k=256):
     dev = "cuda:0"
