@@ -496,6 +496,9 @@ w4a16_tc2_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant_
           const int st = step % S;
           if (step >= first) {
             if (!warp_wait(smem_u32(&bars->empty[st]), ((step / S) & 1) ^ 1, abort, p.wait_ns)) { give_up(p, abort, 15); ok = false; break; }
+          } else if (__any_sync(0xffffffffu, *abort)) {   // (given up while the previous kernel ran: nothing new into a CTA that ends)
+            ok = false;
+            break;
           }
           if (elect_one()) {
             if (step >= first) issue_weights(st, n_idx2, kk);
@@ -505,12 +508,18 @@ w4a16_tc2_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant_
         }
       }
     }
-    if (*abort) {   // unwinding: let this CTA's own weight copies land (activation bytes are counted in the leader)
+    if (*abort) {   // unwinding: let the copies in flight land
       volatile int never = 0;
-      const int issued = step < S ? step : S;
-      for (int i = 0; i < issued; ++i) {
-        const int sidx = step - 1 - i;
-        mbar_wait(smem_u32(&bars->wsfull[sidx % S]), (sidx / S) & 1, &never, 200000000ull);
+      const int issued = max(step, first);
+      for (int i = max(0, issued - S); i < issued; ++i) mbar_wait(smem_u32(&bars->wsfull[i % S]), (i / S) & 1, &never, 200000000ull);
+      if (rank == 0) {
+        // Both CTAs' activation bytes are counted here, and the CTAs leave together.  (200 ms in all: a partner that gave up
+        // before this one has not requested all of these stages.)
+        const uint64_t t0 = globaltimer_ns(), most = 200000000ull;
+        for (int i = max(0, step - S); i < step; ++i) {
+          const uint64_t spent = globaltimer_ns() - t0;
+          mbar_wait(smem_u32(&bars->afull[i % S]), (i / S) & 1, &never, spent < most ? most - spent : 1);
+        }
       }
     }
   } else if (rank == 0) {
