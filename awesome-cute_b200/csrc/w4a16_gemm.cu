@@ -642,7 +642,7 @@ int launch_skinny(const Problem &pr) {
   set_output(p, pr);
   p.wait_ns = pr.wait_ns;
 
-  const int cl = skinny_cluster(MT, p.n_tiles, pr.k, KS, nsm, pr.plan ? nullptr : fit[pr.dev]);
+  const int cl = pr.orphan_finisher ? 1 : skinny_cluster(MT, p.n_tiles, pr.k, KS, nsm, pr.plan ? nullptr : fit[pr.dev]);
   if (cl == 0) return -2;
   int grid = p.n_tiles * cl;
   if (cl == 1) {
@@ -652,6 +652,11 @@ int launch_skinny(const Problem &pr) {
     if (p.n_tiles <= grid) grid = pick_workers(p.n_tiles, p.k_iters, grid, 0.7 * KS / 256, 0.12);
     p.iters_per_cta = (p.total_iters + grid - 1) / grid;
     grid = (p.total_iters + p.iters_per_cta - 1) / p.iters_per_cta;
+  }
+  if (pr.orphan_finisher) {
+    if (p.k_iters < 2) return W4A16_ERR_ARG;
+    p.iters_per_cta = p.k_iters / 2;   // as in launch_single
+    grid = 1;
   }
   if (pr.plan) {   // (in units of two CTAs, one SM's worth)
     const int kernel = cl > 1 ? W4A16_KERNEL_DECODE_CLUSTER : pr.k % 256 == 0 ? W4A16_KERNEL_DECODE : W4A16_KERNEL_SINGLE;
@@ -997,7 +1002,8 @@ int dispatch_tc(const Problem &pr) {
   // 9 to 16 rows: where latency counts, and for k an odd multiple of 128 (m = 16, us: 512 x 2048 5.7 -> 4.1, 512 x 8192
   // 9.1 -> 5.6, 4096 x 1024 5.6 -> 4.5, 1024 x 4480 8.6 -> 5.2; from 8 million weights on the kernels are level).
   const bool few_weights = pr.k <= 8192 && ((long)pr.n * pr.k <= 7000000 || pr.n <= 12 * w4a16::TILE_N);
-  if (pr.m <= (!k256 || few_weights ? 16 : 8) && k128 && g_use_skinny && pr.sms <= 0 && !pr.orphan_finisher) {
+  // (the self-test of the waits runs on this kernel up to 8 rows)
+  if (pr.m <= (pr.orphan_finisher ? 8 : !k256 || few_weights ? 16 : 8) && k128 && g_use_skinny && pr.sms <= 0) {
     const int rc = launch_skinny_g(pr);
     if (rc != -2) return rc;
   }

@@ -248,7 +248,8 @@ __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatil
 }
 
 // Waits for the bytes that st_async of other CTAs of the cluster counts; bounded, but not cut short by an abort: a CTA whose
-// neighbours may still send must not leave.
+// neighbours may still send must not leave.  A CTA that gave up sends too, so this ends soon after the others' own waits; its
+// limit (eight times theirs at the callers) only runs out on a CTA that never comes to send.
 __device__ __forceinline__ bool warp_wait_cluster(uint32_t bar, uint32_t parity, uint64_t limit_ns) {
   const uint64_t t0 = sm100::globaltimer_ns();
   bool ok = false;

@@ -232,7 +232,8 @@ w4a16_tc2_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant_
       sch = p.s[n0 + row - c32 + 8 * ((c32 & 7) >> 1) + 2 * (c32 >> 3) + (c32 & 1)];
     }
     pdl_wait_prior_grid();
-    if (!warp_wait(smem_u32(&bars->accfull[0]), 0, abort, p.wait_ns)) { give_up(p, abort, 13); return; }
+    const bool ok = warp_wait(smem_u32(&bars->accfull[0]), 0, abort, p.wait_ns);
+    if (!ok) give_up(p, abort, 13);
     tc_fence_after();
     const uint32_t t_acc = tmem + ((uint32_t)(quad * 32) << 16);
     float *slab = reinterpret_cast<float *>(reinterpret_cast<uint8_t *>(bars) + Cfg::BAR_BYTES + Cfg::GATHER_BYTES);
@@ -241,7 +242,7 @@ w4a16_tc2_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant_
     for (int c = h; c * 16 < width; c += H) {
       const int owner = c % P;
       if (owner == q) continue;
-      uint32_t v[16];
+      uint32_t v[16];   // (after a give-up whatever is there: the others need not wait for what would never come)
       tmem_ld_32x32b_x16(t_acc + c * 16, v);
       tc_wait_ld();
       const uint32_t to = 2 * owner + rank, slot = (uint32_t)(c / P * (P - 1) + (q < owner ? q : q - 1));
@@ -250,8 +251,9 @@ w4a16_tc2_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant_
       for (int i = 0; i < 16; ++i) st_async_f32(dst + (uint32_t)i * (TILE_N * 4), __uint_as_float(v[i]), dbar);
     }
     const int dests = 1 + p.n_extra + (p.C2 ? 1 : 0);
-    // (longer than any other wait: a CTA that gave up sends nothing, one that did not sends before this ends)
+    // (longer than any other wait: nothing may arrive in a CTA that has left)
     if (q * 16 < width && !warp_wait_cluster(bar_u, 0, 8 * p.wait_ns)) { give_up(p, abort, 14); return; }
+    if (!ok) return;
 #pragma unroll 1
     for (int c = h; c * 16 < width; c += H) {
       if (c % P != q) continue;

@@ -381,17 +381,16 @@ w4a16_decode_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_consta
         // columns, so a warp's 4-byte stores are one 128-byte packet.
         cluster_wait();
         const uint32_t slab_u = smem_u32(xslab) + (uint32_t)row * 4, bar_u = smem_u32(&bars->xfull);
-        if (ok) {
+        // (also after a give-up, whose sums mean nothing: the others need not wait for what would never come)
 #pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            const uint32_t owner = i % CL;
-            if (owner == crank || i >= p.m) continue;
-            const uint32_t slot = (i / CL) * (CL - 1) + (crank < owner ? crank : crank - 1);
-            st_async_f32(map_to_cta(slab_u + slot * (TILE_N * 4), owner), f[i], map_to_cta(bar_u, owner));
-          }
+        for (int i = 0; i < 16; ++i) {
+          const uint32_t owner = i % CL;
+          if (owner == crank || i >= p.m) continue;
+          const uint32_t slot = (i / CL) * (CL - 1) + (crank < owner ? crank : crank - 1);
+          st_async_f32(map_to_cta(slab_u + slot * (TILE_N * 4), owner), f[i], map_to_cta(bar_u, owner));
         }
-        // A rank stays until its rows are complete, also after an abort: nothing may arrive in a CTA that has left.
-        // (Longer than any other wait: a rank that gave up sends nothing, one that did not sends before this ends.)
+        // A rank stays until its rows are complete, also after an abort: nothing may arrive in a CTA that has left.  (Hence a
+        // limit longer than any other.)
         if ((int)crank < p.m && !warp_wait_cluster(bar_u, 0, 8 * p.wait_ns)) { give_up(p, abort, 4); ok = false; }
         if (!ok) break;
         if (warp == NDQ) W4A16_STAMP(7);               // partial rows arrived

@@ -374,8 +374,8 @@ w4a16_skinny_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_consta
         const int slot = (row / cl) * (cl - 1) + (rank < owner ? rank : rank - 1);
         st_async_f4(map_to_cta(smem_u32(slab + slot * TILE_N + 4 * lane), owner), row_sum(row), map_to_cta(smem_u32(&bars->slab), owner));
       }
-      // A rank stays until its rows are complete: nothing may arrive in a CTA that has left.  (A wait longer than any other:
-      // a rank that gave up still sends before this one may leave.)
+      // A rank stays until its rows are complete: nothing may arrive in a CTA that has left.  (Hence a limit longer than any
+      // other; a rank that gave up sends all the same.)
       if (rank < p.m && !warp_wait_cluster(smem_u32(&bars->slab), 0, 8 * p.wait_ns)) { give_up(p, abort, 43); break; }
     }
     // stream-K: CTAs cta + 1 .. cta + pieces hold the rest of a split tile

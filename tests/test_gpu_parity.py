@@ -280,6 +280,67 @@ def test_bounded_wait_runs_out_and_the_stream_survives():
     check(run_mul(At, Bt, st, m, n), orc.c_gemm(A, q, s, gs), "after the timeout")
 
 
+@pytest.mark.parametrize("m,sites", [(5, "44"), (16, "4"), (40, "4 9")])
+def test_bounded_wait_of_each_stream_k_kernel(m, sites):
+    """The same on the kernel that each batch size runs on."""
+    import ctypes
+    import time
+    from awesome_cute_b200 import _lib
+    n, k, gs = 256, 1152, 128
+    A, q, s = orc.make_problem(m, n, k, gs, 56)
+    At, Bt, st = pack_problem(A, q, s)
+    C = torch.zeros((m, n), dtype=torch.half, device=DEV)
+    p = lambda t: ctypes.c_void_p(t.data_ptr())
+    stream = ctypes.c_void_p(torch.cuda.current_stream(0).cuda_stream)
+    run_mul(At, Bt, st, m, n)
+    t0 = time.time()
+    assert _lib.lib.w4a16_selftest_unanswered_wait(p(At), p(Bt), p(C), p(st), m, n, k, gs, 0, stream, 300) == _lib.OK
+    assert _lib.lib.w4a16_device_status(0, stream) == _lib.ERR_TIMEOUT
+    assert _lib.last_cuda_error().split("site ")[1].split()[0] in sites.split()
+    assert 0.25 < time.time() - t0 < 3.0
+    check(run_mul(At, Bt, st, m, n), orc.c_gemm(A, q, s, gs), "after the timeout")
+
+
+def test_clusters_give_up_together():
+    """Kernels in clusters whose waits run out while they wait for the launch before them: every CTA gives up, sends what the
+    others count on all the same, and the launch ends with the one before it, not after the exchange's own, longer limit.
+    The limit is read at load time: a child process."""
+    import os
+    import subprocess
+    import sys
+    code = r"""
+import ctypes, os, sys, time
+sys.path.insert(0, os.getcwd()); sys.path.insert(0, os.path.join(os.getcwd(), 'tests'))
+import torch
+from gpu_common import DEV, check, orc, pack_problem, pkg, run_mul
+L = pkg._lib.lib
+p = lambda t: ctypes.c_void_p(t.data_ptr())
+stream = ctypes.c_void_p(torch.cuda.current_stream(0).cuda_stream)
+blocker = orc.make_problem(16, 256, 2048, 128, 1)
+bA, bB, bs = pack_problem(*blocker)
+bC = torch.zeros((16, 256), dtype=torch.half, device=DEV)
+for m, n, k in ((4, 512, 8192), (16, 4096, 4096), (48, 1024, 8192), (100, 1024, 8192)):
+    A, q, s = orc.make_problem(m, n, k, 128, m)
+    At, Bt, st = pack_problem(A, q, s)
+    want = run_mul(At, Bt, st, m, n)
+    C = torch.zeros((m, n), dtype=torch.half, device=DEV)
+    ws = torch.zeros(n // 128 * 16, dtype=torch.int, device=DEV)
+    torch.cuda.synchronize()
+    t0 = time.time()
+    assert L.w4a16_selftest_unanswered_wait(p(bA), p(bB), p(bC), p(bs), 16, 256, 2048, 128, 0, stream, 700) == 0
+    pkg.mul(At, Bt, C, st, ws)
+    assert L.w4a16_device_status(0, stream) == pkg._lib.ERR_TIMEOUT
+    took = time.time() - t0
+    assert 0.6 < took < 1.2, (m, took)
+    assert torch.equal(run_mul(At, Bt, st, m, n), want)
+print('ok')
+"""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", code], cwd=root, env=dict(os.environ, W4A16_WAIT_MS="150"), capture_output=True, text=True,
+                       timeout=300)
+    assert r.returncode == 0 and "ok" in r.stdout, r.stdout[-2000:] + r.stderr[-2000:]
+
+
 @pytest.mark.parametrize("m", [16, 256])
 def test_dependent_chain_eager_and_graph_replay(m):
     """Consecutive GEMMs on one stream where each one's output is the next one's activations: the next kernel
