@@ -25,6 +25,7 @@ SYMBOLS = {
     "w4a16_device_status": (_i, [_i, _vp]),
     "w4a16_release_stream": (_i, [_i, _vp]),
     "w4a16_plan": (_i, [_i, _i, _i, _i, _i, _i, _vp]),
+    "w4a16_plan_kernel": (ctypes.c_char_p, [_i, _i, _i, _i, _i, _i]),
     "w4a16_selftest_unanswered_wait": (_i, [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _vp, _i]),
     "w4a16_last_cuda_error": (ctypes.c_char_p, []),
     "w4a16_pack_weights": (_i, [_vp, _i, _i, _vp]),
@@ -95,6 +96,11 @@ def plan(m, n, k, groupsize=128, sms=-1, device_sms=148):
     d = {f: getattr(out, f) for f, _ in Plan._fields_}
     d["kernel"] = KERNEL_NAMES.get(d["kernel"], d["kernel"])
     return rc, d
+
+
+def plan_kernel(m, n, k, groupsize=128, sms=-1, device_sms=148):
+    """The name of that kernel and the size of its clusters, "" where none would be launched (w4a16_plan_kernel)."""
+    return lib.w4a16_plan_kernel(m, n, k, groupsize, sms, device_sms).decode()
 
 
 def last_cuda_error():

@@ -187,12 +187,19 @@ struct Problem {
   // set only by w4a16_plan: describe the launch instead of making it (no CUDA call on that path)
   w4a16_plan_t *plan = nullptr;
   int plan_sms = 0;                 // SMs of the device the plan is for
+  std::string *plan_kernel = nullptr;   // set only by w4a16_plan_kernel
 };
 
 // SMs of the problem's device: asked of CUDA, or given by the caller of w4a16_plan
 int problem_sm_count(const Problem &pr);
 
 int problem_sm_count(const Problem &pr) { return pr.plan ? pr.plan_sms : sm_count(pr.dev); }
+
+int planned(const Problem &pr, const w4a16_plan_t &plan, const char *kernel, int cluster = 1, const char *unit = "") {
+  *pr.plan = plan;
+  if (pr.plan_kernel) *pr.plan_kernel = cluster > 1 ? std::string(kernel) + " in clusters of " + std::to_string(cluster) + unit : kernel;
+  return W4A16_OK;
+}
 
 void set_output(w4a16::Params &p, const Problem &pr) {
   p.C = static_cast<__half *>(pr.C);
@@ -408,8 +415,8 @@ int launch_single(const Problem &pr) {
   }
 
   if (pr.plan) {
-    *pr.plan = w4a16_plan_t{K::IS_DECODE ? W4A16_KERNEL_DECODE : W4A16_KERNEL_SINGLE, K::TM, K::KS, grid, 1, 0, p.iters_per_cta};
-    return W4A16_OK;
+    return planned(pr, {K::IS_DECODE ? W4A16_KERNEL_DECODE : W4A16_KERNEL_SINGLE, K::TM, K::KS, grid, 1, 0, p.iters_per_cta},
+                   K::IS_DECODE ? "w4a16_decode_kernel" : "w4a16_tc_kernel");
   }
   Maps mp;
   if (!get_maps(pr, K::KS, K::TM, K::GROUPED, K::OUT == w4a16::OUT_TMA, mp)) return W4A16_ERR_CUDA;
@@ -480,8 +487,8 @@ int launch_decode_cluster(const Problem &pr) {
   if (nsm <= 0) return W4A16_ERR_CUDA;
   if (pr.plan) {   // (as if every cluster of this size could be resident: a cluster lives inside one GPC)
     if (nsm / CL < pr.n / w4a16::TILE_N) return -2;
-    *pr.plan = w4a16_plan_t{W4A16_KERNEL_DECODE_CLUSTER, Cfg::TM, Cfg::KS, pr.n / w4a16::TILE_N * CL, CL, 0, pr.k / Cfg::KS / CL};
-    return W4A16_OK;
+    return planned(pr, {W4A16_KERNEL_DECODE_CLUSTER, Cfg::TM, Cfg::KS, pr.n / w4a16::TILE_N * CL, CL, 0, pr.k / Cfg::KS / CL},
+                   "w4a16_decode_kernel", CL);
   }
   w4a16::Params p{};
   p.m = pr.m, p.n = pr.n, p.k = pr.k;
@@ -660,8 +667,8 @@ int launch_skinny(const Problem &pr) {
   }
   if (pr.plan) {   // (in units of two CTAs, one SM's worth)
     const int kernel = cl > 1 ? W4A16_KERNEL_DECODE_CLUSTER : pr.k % 256 == 0 ? W4A16_KERNEL_DECODE : W4A16_KERNEL_SINGLE;
-    *pr.plan = w4a16_plan_t{kernel, 16, KS, (grid + 1) / 2, cl > 1 ? cl / 2 : 2, 0, cl > 1 ? p.k_iters / (cl / 2) : 2 * p.iters_per_cta};
-    return W4A16_OK;
+    return planned(pr, {kernel, 16, KS, (grid + 1) / 2, cl > 1 ? cl / 2 : 2, 0, cl > 1 ? p.k_iters / (cl / 2) : 2 * p.iters_per_cta},
+                   "w4a16_skinny_kernel", cl);
   }
   Maps mp;
   if (!get_maps(pr, KS, Cfg::ROWS, GROUPED, false, mp, true)) return W4A16_ERR_CUDA;
@@ -739,8 +746,7 @@ int launch_tc2_cluster(const Problem &pr) {
   if (p.iters_per_cta * (P - 1) >= p.k_iters) return -2;   // (a pair without a stage)
   if (pr.plan) {
     if (2 * P * tiles > nsm) return -2;
-    *pr.plan = w4a16_plan_t{W4A16_KERNEL_PAIRS, TM, Cfg::KS, p.workers, 2, 0, p.iters_per_cta};
-    return W4A16_OK;
+    return planned(pr, {W4A16_KERNEL_PAIRS, TM, Cfg::KS, p.workers, 2, 0, p.iters_per_cta}, "w4a16_tc2_kernel", P, " pairs");
   }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(2 * P * tiles));
@@ -928,8 +934,7 @@ int launch_tc2(const Problem &pr) {
   if (p.dp_waves == 0) pairs = (p.total_iters + p.iters_per_cta - 1) / p.iters_per_cta;
   p.workers = pairs;
   if (pr.plan) {
-    *pr.plan = w4a16_plan_t{W4A16_KERNEL_PAIRS, TM, Cfg::KS, pairs, 2, p.dp_waves, p.total_iters > 0 ? p.iters_per_cta : 0};
-    return W4A16_OK;
+    return planned(pr, {W4A16_KERNEL_PAIRS, TM, Cfg::KS, pairs, 2, p.dp_waves, p.total_iters > 0 ? p.iters_per_cta : 0}, "w4a16_tc2_kernel");
   }
   cfg.gridDim = dim3((unsigned)(2 * pairs));
   Maps mp;   // each CTA of the pair loads half of the tile's activation rows
@@ -1197,7 +1202,8 @@ extern "C" int w4a16_marlin_gemm(const void *A, const void *B, void *C, const vo
                     static_cast<cudaStream_t>(stream), thread_k, thread_n, sms, max_par);
 }
 
-extern "C" int w4a16_plan(int prob_m, int prob_n, int prob_k, int groupsize, int sms, int device_sms, w4a16_plan_t *out) {
+namespace {
+int plan_entry(int prob_m, int prob_n, int prob_k, int groupsize, int sms, int device_sms, w4a16_plan_t *out, std::string *kernel) {
   if (!out || device_sms < 2 || device_sms > MAX_GRID || prob_m < 0 || prob_n < 0 || prob_k < 0) return W4A16_ERR_ARG;
   int thread_k = -1, thread_n = -1;
   const int chk = check_problem(prob_m, prob_n, prob_k, groupsize, thread_k, thread_n);
@@ -1207,7 +1213,21 @@ extern "C" int w4a16_plan(int prob_m, int prob_n, int prob_k, int groupsize, int
   Problem pr{nullptr, nullptr, nullptr, nullptr, prob_m, prob_n, prob_k, groupsize, 0, sms, nullptr};
   pr.plan = out;
   pr.plan_sms = device_sms;
+  pr.plan_kernel = kernel;
   return dispatch_tc(pr);
+}
+}  // namespace
+
+extern "C" int w4a16_plan(int prob_m, int prob_n, int prob_k, int groupsize, int sms, int device_sms, w4a16_plan_t *out) {
+  return plan_entry(prob_m, prob_n, prob_k, groupsize, sms, device_sms, out, nullptr);
+}
+
+extern "C" const char *w4a16_plan_kernel(int prob_m, int prob_n, int prob_k, int groupsize, int sms, int device_sms) {
+  static thread_local std::string kernel;
+  w4a16_plan_t plan;
+  kernel.clear();
+  plan_entry(prob_m, prob_n, prob_k, groupsize, sms, device_sms, &plan, &kernel);
+  return kernel.c_str();
 }
 
 // The GEMM with HOST activations and HOST output: copy in, multiply, copy out, all enqueued on `stream`.

@@ -172,9 +172,11 @@ int w4a16_device_status(int dev, void *stream);
 #define W4A16_KERNEL_PAIRS 2          /* one CTA pair per worker (256 weight columns per tile) */
 #define W4A16_KERNEL_DECODE 3         /* prob_m <= 16: one CTA per worker, stream-K or one whole tile each */
 #define W4A16_KERNEL_DECODE_CLUSTER 4 /* prob_m <= 16: one cluster per 128-column tile */
-/* prob_m <= 8 without an explicit `sms`, and some problems of up to 16 rows, run on CTAs that take half an SM; a pair of
- * them counts as one below (a worker is two CTAs; `workers` of the cluster form and the cluster size count pairs).
- * tile_rows is 16 there too: at prob_m <= 8 the tile's room is 8. */
+/* prob_m <= 8 without an explicit `sms`, and some problems of up to 16 rows, run on the mma.sync kernel, whose CTAs take half an
+ * SM.  It has no code of its own (a caller compiled before it keeps reading what it knows): it is reported as DECODE or
+ * DECODE_CLUSTER, or as SINGLE for k an odd multiple of 128, with a pair of its CTAs counted as one below (a worker is two
+ * CTAs; `workers` of the cluster form and the cluster size count pairs) and tile_rows 16, although at prob_m <= 8 the tile's
+ * room is 8.  w4a16_plan_kernel names the kernel itself. */
 typedef struct {
   int kernel;            /* W4A16_KERNEL_* */
   int tile_rows;         /* batch rows per tile */
@@ -185,6 +187,9 @@ typedef struct {
   int stages_per_worker; /* k-stages per worker in the stream-K part (the cluster form: per CTA) */
 } w4a16_plan_t;
 int w4a16_plan(int prob_m, int prob_n, int prob_k, int groupsize, int sms, int device_sms, w4a16_plan_t *out);
+/* The name of that kernel, with the size of its clusters where it runs in clusters ("w4a16_skinny_kernel in clusters of 8",
+ * "w4a16_tc2_kernel in clusters of 3 pairs"); "" where the call would launch none.  Valid until the thread's next call. */
+const char *w4a16_plan_kernel(int prob_m, int prob_n, int prob_k, int groupsize, int sms, int device_sms);
 
 /* Frees the scratch and status word the library keeps for (dev, stream), after synchronising `stream`.  No launch
  * captured in a CUDA graph on that stream may be replayed afterwards.  The reference has no counterpart (it owns

@@ -121,3 +121,21 @@ def test_every_plan_covers_its_problem():
             assert (d["kernel"] == "decode") == (m <= 16 and k % 256 == 0)
             assert w * per >= tiles * k_iters, (m, n, k, d)
             assert (w - 1) * per < tiles * k_iters, (m, n, k, d)      # no worker without work
+
+
+def test_the_kernel_by_name():
+    """w4a16_plan reports the mma.sync kernel under the codes of the kernels before it; the name tells them apart."""
+    name = lambda *a, **kw: pkg.plan_kernel(*a, **kw).replace("w4a16_", "").replace("_kernel", "")
+    # up to 8 rows, and small layers or odd multiples of 128 up to 16
+    assert name(1, 4096, 4096) == name(8, 4096, 4096, -1) == "skinny in clusters of 8"
+    assert name(8, 22016, 4096) == name(1, 8192, 28672) == "skinny"
+    assert name(16, 512, 2048) == "skinny in clusters of 8" and name(16, 12288, 4224) == "skinny"
+    assert name(8, 4096, 4096, sms=37) == "decode"
+    # the tcgen05 kernels
+    assert name(16, 4096, 4096) == "decode in clusters of 4" and name(9, 8192, 8192) == "decode in clusters of 2"
+    assert name(16, 12288, 4096) == name(16, 22016, 4096) == "decode"
+    assert name(16, 4096, 4224) == name(24, 4096, 4224) == name(128, 4096, 512) == "tc"
+    assert name(24, 4096, 4096) == "tc2 in clusters of 2 pairs" and name(77, 5120, 5504, -1) == "tc2 in clusters of 3 pairs"
+    assert name(48, 1024, 8192) == "tc2 in clusters of 4 pairs"
+    assert name(48, 22016, 4096) == name(4096, 57344, 8192) == "tc2"
+    assert name(0, 4096, 4096) == name(16, 4100, 4096) == ""
