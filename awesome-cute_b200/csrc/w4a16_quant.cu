@@ -140,7 +140,7 @@ extern "C" int w4a16_quantize_pack_device(const void *weight_nk, const void *sca
   const int group = groupsize == -1 ? k : groupsize;
   const int groups = k / group;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (reinterpret_cast<uintptr_t>(weight_nk) & 15) return W4A16_ERR_ARG;   // rows are read 16 bytes at a time (k % 128 == 0)
+  if (reinterpret_cast<uintptr_t>(weight_nk) & 15) return W4A16_ERR_ARG;   // the library's alignment of operands (rows are read 8 bytes at a time)
   quantize_pack_kernel<<<dim3((unsigned)((k / PACK_K + PACK_THREADS / 32 - 1) / (PACK_THREADS / 32)), (unsigned)(n / 64)), PACK_THREADS, 0, st>>>(
       static_cast<const __half *>(weight_nk), static_cast<const __half *>(scales), k, n, group, groups,
       !(reinterpret_cast<uintptr_t>(B) & 15), static_cast<uint32_t *>(B), static_cast<__half *>(s_packed));

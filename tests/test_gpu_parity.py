@@ -544,6 +544,29 @@ def test_device_quantize_pack_edges(n, k, groupsize):
     assert np.array_equal(sp_dev.cpu().numpy().view(np.uint16), sp_host.view(np.uint16))
 
 
+def test_device_quantize_pack_beside_quotients_that_overflow():
+    """A word with a quotient beyond fp16 is redone weight by weight: its other weights, and every other word, come out as on the
+    host.  (What becomes of the quotient itself the host's float-to-int conversion leaves open.)"""
+    k, n, groupsize = 256, 512, 128
+    rng = np.random.default_rng(8)
+    s = rng.uniform(0.005, 0.02, size=(k // groupsize, n)).astype(np.float16)
+    w = (rng.integers(-24, 25, size=(n, k)) * 0.5 * np.repeat(s.astype(np.float32).T, groupsize, axis=1)).astype(np.float16)
+    tiny = np.arange(0, n, 7)                   # columns of a scale so small that most quotients overflow, some zero, some finite
+    s[:, tiny] = np.float16(2.0 ** -23)
+    w[tiny] = (rng.choice([-1, 0, 1, 2.0 ** -22, -2.0 ** -21, 3 * 2.0 ** -23], size=(len(tiny), k))).astype(np.float16)
+    lone = rng.integers(0, n, size=64)          # and lone weights that overflow among ordinary ones
+    w[lone, rng.integers(0, k, size=64)] = rng.choice([-65504, 65504], size=64).astype(np.float16)
+    quotient = w.astype(np.float32) / np.repeat(s.astype(np.float32).T, groupsize, axis=1)
+    with np.errstate(over="ignore"):
+        defined = np.isfinite(quotient.astype(np.float16)).T
+    assert 0.02 < 1 - defined.mean() < 0.2
+    B_host, sp_host = pkg.quantize_pack(w, s, groupsize)
+    B_dev, sp_dev = pkg.quantize_pack_device(to_dev(w), to_dev(s), groupsize)
+    assert np.array_equal(sp_dev.cpu().numpy().view(np.uint16), sp_host.view(np.uint16))
+    q_host, q_dev = pkg.unpack_weights(B_host, k, n), pkg.unpack_weights(B_dev.cpu().numpy(), k, n)
+    assert np.array_equal(q_dev[defined], q_host[defined])
+
+
 @pytest.mark.parametrize("m,n,k,groupsize", [
     (17, 512, 1024, 128), (33, 1024, 8192, -1), (64, 512, 768, 128), (40, 2048, 2816, 128), (24, 4096, 4096, -1),   # 256-k stages
     (77, 5120, 5504, -1), (80, 1024, 2048, 128), (129, 512, 8192, 128), (190, 256, 1536, 128), (500, 512, 6272, -1), (100, 2048, 8192, 128)])
