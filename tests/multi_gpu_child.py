@@ -16,16 +16,10 @@ import __graft_entry__ as entry  # noqa: E402
 from oracle import oracle as orc  # noqa: E402
 
 
-def main():
-    rank, world = int(os.environ["RANK"]), int(os.environ["WORLD_SIZE"])
-    torch.cuda.set_device(rank)
-    dev = torch.device("cuda", rank)
-    dist.init_process_group("gloo")
-    pkg = entry.load_package()
-    n, k, gs = 512 * world, 1024, 128
+def run(pkg, dev, rank, world, n, k, batches, gs=128):
     bufs = [pkg.GatherBuffers(1024, n, rank, world, dev) for _ in range(2)]     # alternate: no write-after-read hazard
     bad = 0
-    for it, m in enumerate((16, 300, 1024, 16)):
+    for it, m in enumerate(batches):
         A, q, s = orc.make_problem(m, n, k, gs, 100 + it)                      # same on every rank
         layer = pkg.ColumnShardedLayer(pkg.pack_weights(q), pkg.permute_scales(s), rank, world, dev)
         out = layer.forward_gathered(torch.from_numpy(A).to(dev), bufs[it % 2])
@@ -42,6 +36,19 @@ def main():
             bad += 1
     for b in bufs:
         b.close()
+    return bad
+
+
+def main():
+    rank, world = int(os.environ["RANK"]), int(os.environ["WORLD_SIZE"])
+    torch.cuda.set_device(rank)
+    dev = torch.device("cuda", rank)
+    dist.init_process_group("gloo")
+    pkg = entry.load_package()
+    bad = 0
+    # columns per rank and k: small problems (mma.sync kernel, clusters of CTA pairs), and some that keep to the decode kernel
+    for n_local, k, batches in ((512, 1024, (16, 300, 1024, 16)), (4096, 2048, (16, 9, 40, 16))):
+        bad += run(pkg, dev, rank, world, n_local * world, k, batches)
     verdict = torch.tensor([bad])
     dist.all_reduce(verdict)
     dist.destroy_process_group()

@@ -341,12 +341,16 @@ print('ok')
     assert r.returncode == 0 and "ok" in r.stdout, r.stdout[-2000:] + r.stderr[-2000:]
 
 
-@pytest.mark.parametrize("m", [16, 256])
-def test_dependent_chain_eager_and_graph_replay(m):
+@pytest.mark.parametrize("m,dims,kernel", [
+    (16, [1024, 2048, 1024, 512], "skinny"), (256, [1024, 2048, 1024, 512], "tc2"), (5, [1024, 19200, 1152], "skinny"),
+    (16, [4096, 4096, 2048, 4096], "decode"), (12, [1024, 19200, 1024], "decode"), (40, [1024, 2048, 1024], "tc2"),
+    (40, [1152, 1024, 512], "tc")])
+def test_dependent_chain_eager_and_graph_replay(m, dims, kernel):
     """Consecutive GEMMs on one stream where each one's output is the next one's activations: the next kernel
     may start early (programmatic dependent launch) but must not read its activations, write C or touch the
     scratch before the previous kernel has finished.  Checked eagerly and over several CUDA-graph replays."""
-    dims, gs = [1024, 2048, 1024, 512], 128
+    gs = 128
+    assert pkg.plan_kernel(m, dims[1], dims[0]).startswith("w4a16_%s_kernel" % kernel)
     rng = np.random.default_rng(91)
     A0 = (rng.standard_normal((m, dims[0]), dtype=np.float32) * 0.5).astype(np.float16)
     layers = []
@@ -674,6 +678,39 @@ def test_host_calls_that_share_buffers(m, d):
         assert torch.equal(h[5].to(DEV), mul(h[4], 5))
 
 
+@pytest.mark.parametrize("m,n,k,gs,kernel", [
+    (16, 4096, 4096, 128, "decode_kernel in clusters of 4"), (9, 4096, 11008, -1, "decode_kernel in clusters of 4"),
+    (16, 8192, 1024, -1, "decode_kernel in clusters of 2"), (13, 2048, 4096, 128, "decode_kernel in clusters of 8"),
+    (16, 12288, 1024, 128, "decode_kernel"), (16, 19200, 1024, -1, "decode_kernel"), (11, 5120, 5120, 128, "decode_kernel"),
+    (8, 4096, 4096, 128, "skinny_kernel in clusters of 8"), (3, 19200, 1024, -1, "skinny_kernel"), (16, 12288, 1152, 128, "skinny_kernel"),
+    (24, 512, 1152, 128, "tc_kernel"), (40, 512, 1152, -1, "tc_kernel"), (96, 512, 640, 128, "tc_kernel"),
+    (20, 19456, 512, 128, "tc2_kernel"), (40, 19456, 512, -1, "tc2_kernel"), (96, 19456, 1024, 128, "tc2_kernel"),
+    (20, 1024, 2048, 128, "tc2_kernel in clusters of 4 pairs"), (77, 5120, 5504, -1, "tc2_kernel in clusters of 3 pairs")])
+def test_host_output_of_each_kernel(m, n, k, gs, kernel):
+    """The instantiations that write to host memory as well: C_host and C_stage are mul()'s result bit for bit, also when the
+    call is made again on the same buffers and other activations."""
+    assert pkg.plan_kernel(m, n, k, gs) == "w4a16_" + kernel
+    gen = torch.Generator(device=DEV).manual_seed(m + n + k)
+    B = torch.randint(-2 ** 31, 2 ** 31, (k // 16, 2 * n), generator=gen, device=DEV, dtype=torch.int)
+    s = (torch.rand((1 if gs == -1 else k // gs, n), generator=gen, device=DEV) * 0.015 + 0.005).half()
+    ws = torch.zeros(n // 128 * 16, dtype=torch.int, device=DEV)
+    A = torch.zeros((m, k), dtype=torch.half).pin_memory()
+    C = torch.zeros((m, n), dtype=torch.half).pin_memory()
+    sa, sc = torch.zeros((m, k), dtype=torch.half, device=DEV), torch.zeros((m, n), dtype=torch.half, device=DEV)
+    op = pkg.HostGemm(A, B, C, s, ws, sa, sc)
+    op()                        # (the first call on a stream may go through the copy engines)
+    for _ in range(3):
+        torch.cuda.synchronize()
+        A.copy_(torch.randn((m, k), generator=gen, device=DEV).half())
+        C.fill_(float("nan"))
+        sc.fill_(float("nan"))
+        op()
+        pkg.device_status(0)
+        want = torch.zeros((m, n), dtype=torch.half, device=DEV)
+        pkg.mul(A.to(DEV), B, want, s, ws)
+        assert torch.equal(sc, want) and torch.equal(C.to(DEV), want)
+
+
 @pytest.mark.parametrize("m", [4, 40])
 def test_captured_host_calls_between_eager_ones(m):
     """Calls with host buffers in a CUDA graph, replayed between eager ones on the same stream and the same staging buffers."""
@@ -775,6 +812,9 @@ def test_pair_kernel_dependent_chain_graph_replay():
 
 @pytest.mark.parametrize("m,nl,k,gs", [(16, 512, 1024, 128), (48, 256, 2048, 128), (200, 512, 512, 128),
                                        (1024, 2048, 4096, 128), (33, 512, 1024, -1), (7, 256, 256, -1),
+                                       (16, 4096, 2048, 128), (9, 4096, 4096, -1), (13, 19200, 512, 128),   # decode kernel
+                                       (40, 512, 1152, 128), (128, 512, 640, -1),       # general kernel, 64- and 128-row tiles
+                                       (40, 19456, 512, 128),        # CTA pairs, 64-row tiles, without clusters
                                        (1024, 4096, 4096, 128),      # CTA pairs, 128-row tiles
                                        (960, 4096, 4096, -1)])       # CTA pairs, 192-row tiles, per-channel scales
 def test_gathering_epilogue_on_one_gpu(m, nl, k, gs):

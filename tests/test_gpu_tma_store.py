@@ -21,14 +21,20 @@ sys.path.insert(0, os.getcwd()); sys.path.insert(0, os.path.join(os.getcwd(), 't
 import numpy as np, torch
 from gpu_common import orc, pkg, pack_problem, run_mul, check
 cases = [
-    # decode kernel: ragged rows, stream-K and cluster forms, both scale kinds
+    # decode kernel, whole tiles and stream-K (clusters, and the mma.sync kernel of small problems, always store from registers:
+    # they are here for the comparison with the oracle; an explicit split keeps a problem off them)
+    (3, 512, 1024, 128, 4), (16, 512, 2048, -1, 9), (1, 4096, 4096, 128, 100), (12, 4096, 2048, -1, 148), (16, 19200, 512, 128, -1),
     (3, 512, 1024, 128, -1), (16, 512, 2048, -1, -1), (1, 4096, 4096, 128, -1), (12, 4096, 2048, -1, -1), (16, 12288, 1024, 128, -1),
     (16, 512, 2048, 128, 7),
-    # general kernel: 17..64 rows with an explicit split, 128- and 192-row tiles, ragged, per-channel
+    # general kernel: 17..64 rows, 128-row tiles, ragged, per-channel
+    (24, 512, 1152, 128, 5), (40, 512, 1152, -1, -1), (118, 512, 640, 128, -1), (200, 512, 640, -1, -1),
+    # CTA pairs of each batch tile, with an explicit split
     (24, 512, 1024, 128, 5), (64, 256, 2048, -1, 9), (118, 512, 1024, 128, -1), (118, 256, 512, -1, -1), (200, 512, 1024, 128, 11),
-    # CTA pairs: 33..64 rows, and batches past 128 rows with a ragged last tile
-    (48, 512, 4096, 128, -1), (577, 4096, 8192, 128, -1), (577, 1024, 8192, -1, -1),
+    # CTA pairs: 33..64 rows (also in clusters), and batches past 128 rows with a ragged last tile
+    (48, 512, 4096, 128, 8), (20, 19456, 512, -1, -1), (48, 512, 4096, 128, -1), (577, 4096, 8192, 128, -1), (577, 1024, 8192, -1, -1),
 ]
+staged = [c for c in cases if "skinny" not in pkg.plan_kernel(*c) and "clusters" not in pkg.plan_kernel(*c)]
+assert {pkg.plan_kernel(*c) for c in staged} == {"w4a16_decode_kernel", "w4a16_tc_kernel", "w4a16_tc2_kernel"} and len(staged) >= 16
 digest = hashlib.sha256()
 for (m, n, k, gs, sms) in cases:
     A, q, s = orc.make_problem(m, n, k, gs, seed=m + n + k)
