@@ -791,12 +791,18 @@ const bool g_use_pair_cluster = [] {
 }();
 
 // How many pairs work on a tile when there are fewer tiles than pairs, cheapest first, and 0 for the stream-K form with the
-// worker count of pick_workers.  Priced like that (a stage 0.45 us); what a cluster costs beside its stages hardly depends
-// on the tile, 0.3 us per further pair up to 64 rows and 0.7 us above, until clusters of six and eight CTAs take more than about
-// 90 SMs: they then wait for the previous launch to leave enough SMs of one GPC (1.5 us at 32 rows, 2.5 at 64, 2 above).  The
-// stream-K form pays its partial tiles and 3 us (1.5 above 64 rows, where every piece is priced at 2.2).  Above 64 rows a pair
-// keeps at least 12 stages unless pick_workers cuts shorter.  The limits on the SMs are what fits on 148 (clusters of 4 / 6 / 8:
-// 37 / 20 / 12 or more).  Measured, us, stream-K -> clusters: m = 24: 4096 x 4096 9.4 -> 7.2 (P = 2), 2048 x 8192 10.7 -> 8.6 (4),
+// worker count of pick_workers.  A model fitted to the launches below, not derived.  A stage costs 0.45 us as there; what a
+// cluster costs beside its stages hardly depends on the tile, 0.3 us per further pair up to 64 rows and 0.7 us above, until
+// clusters of six and eight CTAs take more than about 90 SMs: they then wait for the previous launch to leave enough SMs of one
+// GPC (1.5 us at 32 rows, 2.5 at 64, 2 above).  The stream-K form pays its partial tiles and 3 us (1.5 above 64 rows, where every
+// piece is priced at 2.2; up to 64 rows a piece is 0.3 beside those 3 us, where pick_workers, which only compares cuts, has 0.5).
+// Where it takes whole tiles it pays neither, and a cluster on more than half of the SMs (0.6 at 64 rows) costs more than the
+// stages it saves: m = 24, us, whole tiles / clusters of 2: 4096 x 512 4.27 / 3.75, 5632 x 512 4.27 / 4.60, 7168 x 768 4.67 / 5.55;
+// m = 48: 5632 x 768 5.28 / 5.07, 7168 x 512 5.02 / 5.47.
+// Above 64 rows a pair keeps at least 12 stages unless pick_workers cuts shorter; that line was drawn without a measurement, and
+// over 70 random problems of 65 to 1024 rows dropping it is 5 % faster in the mean and nowhere 1 % slower.
+// The shares of the SMs keep w4a16_plan near what fits on 148 (clusters of 4 / 6 / 8: 37 / 20 / 12 or more); the launch itself
+// asks the occupancy call.  Measured, us, stream-K -> clusters: m = 24: 4096 x 4096 9.4 -> 7.2 (P = 2), 2048 x 8192 10.7 -> 8.6 (4),
 // 1024 x 2048 6.5 -> 4.2 (4); m = 48: 1024 x 8192 9.5 -> 7.5 (4); m = 77: 5120 x 5504 14.7 -> 12.0 (3); m = 128: 4096 x 4096
 // 13.7 -> 11.2 (2), 4096 x 11008 21.4 -> 18.5 (3); m = 512: 1024 x 28672 38.5 -> 35.1 (4).
 std::array<int, 3> pick_pair_clusters(int tm, int tiles, int k_iters, int pairs, int nsm) {
@@ -808,7 +814,8 @@ std::array<int, 3> pick_pair_clusters(int tm, int tiles, int k_iters, int pairs,
   std::array<std::pair<double, int>, 3> c;
   for (int P = 2; P <= 4; ++P) {
     const int ctas = 2 * P * tiles, share = (k_iters + P - 1) / P;
-    const bool fits = 100 * ctas <= (P == 2 ? 100 : P == 3 ? 82 : 66) * nsm && share * (P - 1) < k_iters;
+    const int most = pieces == 1 && tm <= 64 ? (tm == 64 ? 60 : 50) : P == 2 ? 100 : P == 3 ? 82 : 66;   // % of the SMs
+    const bool fits = 100 * ctas <= most * nsm && share * (P - 1) < k_iters;
     double cost = 0.45 * share + (P - 2) * (tm >= 128 ? 0.7 : 0.3);
     if (P > 2 && 100 * ctas > 60 * nsm) cost += tm >= 128 ? 2.0 : tm == 64 ? 2.5 : 1.5;
     if (!fits || cost >= stream_k || (tm >= 128 && share < 12 && P != pieces)) cost = 1e9;

@@ -138,4 +138,6 @@ def test_the_kernel_by_name():
     assert name(24, 4096, 4096) == "tc2 in clusters of 2 pairs" and name(77, 5120, 5504, -1) == "tc2 in clusters of 3 pairs"
     assert name(48, 1024, 8192) == "tc2 in clusters of 4 pairs"
     assert name(48, 22016, 4096) == name(4096, 57344, 8192) == "tc2"
+    # two or three stages in all: clusters on up to half of the SMs, whole tiles beyond
+    assert name(24, 4096, 512) == "tc2 in clusters of 2 pairs" and name(24, 5632, 768) == name(48, 7168, 512) == "tc2"
     assert name(0, 4096, 4096) == name(16, 4100, 4096) == ""
