@@ -489,7 +489,7 @@ w4a16_tc2_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant_
     {
       Walk<P> walk(p, pair);
       int tile, kb, ke;
-      bool ok = true;
+      bool ok = !__any_sync(0xffffffffu, *abort);   // (given up while the previous kernel ran: nothing new into a CTA that ends)
       while (ok && walk.next(tile, kb, ke)) {
         int n_idx2, m_idx;
         tile_nm(p, tile, n_idx2, m_idx);
@@ -498,9 +498,6 @@ w4a16_tc2_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant_
           const int st = step % S;
           if (step >= first) {
             if (!warp_wait(smem_u32(&bars->empty[st]), ((step / S) & 1) ^ 1, abort, p.wait_ns)) { give_up(p, abort, 15); ok = false; break; }
-          } else if (__any_sync(0xffffffffu, *abort)) {   // (given up while the previous kernel ran: nothing new into a CTA that ends)
-            ok = false;
-            break;
           }
           if (elect_one()) {
             if (step >= first) issue_weights(st, n_idx2, kk);
