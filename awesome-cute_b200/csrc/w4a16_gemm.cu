@@ -1039,7 +1039,7 @@ int dispatch_tc(const Problem &pr) {
   // 17..32 rows on CTA pairs as well (+12-16 % over the general kernel).  The decode kernel widened to 32- and 64-row
   // tiles (two dequant sets: the accumulator sets need the third operand buffer's tensor-memory columns) was measured
   // 5 % slower than the pairs at 32 rows and 50-90 % slower at 64 (4096 x 4096: 9.6 / 17.9 us against 9.1 / 10.0 us):
-  // at N = 64 its sixteen MMAs per stage take 1024 tensor clocks on ONE SM, the pair spreads them over two.
+  // at N = 64 its sixteen MMAs per stage take 512 tensor clocks (32 each) on ONE SM, the pair spreads them over two.
   if (g_use_pairs && pr.m > 16 && pr.m <= 32 && k256 && pr.n % 256 == 0 && !pr.fixed_partials && !pr.orphan_finisher) {
     const int rc = launch_tc2_g<32, 256>(pr);
     if (rc != -2) return rc;
@@ -1390,7 +1390,7 @@ extern "C" int w4a16_marlin_gemm_simt(const void *A, const void *B, void *C, con
 // Scratch of the stream-K fix-up as a file-scope device array: it exists as soon as the library is loaded on a
 // device (5 MiB of every GPU that loads it, until the process exits) and is shared by every call.
 constexpr int BUILTIN_MAX_M = 64;                                    // batch rows (partial tiles are TM <= 64 wide)
-constexpr size_t BUILTIN_SLOTS = (size_t)160 * BUILTIN_MAX_M * w4a16::TILE_N;   // up to 160 CTAs: 1 310 720 slots
+constexpr size_t BUILTIN_SLOTS = (size_t)160 * BUILTIN_MAX_M * w4a16::TILE_N;   // 160 CTAs' partial tiles of 64 rows: 1 310 720 slots
 static __device__ __align__(256) uint32_t g_builtin_partials[BUILTIN_SLOTS];
 static __device__ __align__(256) int g_builtin_status;
 

@@ -43,7 +43,7 @@ namespace w4a16 {
 
 constexpr int TILE_N = 128;                         // weight columns per tile = UMMA M
 constexpr int EPI_WARPS = 4;
-constexpr uint64_t WAIT_LIMIT_NS = 2000000000ull;   // every device-side wait gives up after 2 s
+constexpr uint64_t WAIT_LIMIT_NS = 2000000000ull;   // every device-side wait gives up after 2 s (see also warp_wait_cluster)
 constexpr int STATUS_TIMEOUT = 4;                   // == W4A16_ERR_TIMEOUT
 constexpr uint32_t PARTIAL_IDLE = 0xffffffffu;      // idle state of a partial-tile slot (a NaN never stored as data)
 

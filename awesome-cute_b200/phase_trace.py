@@ -6,7 +6,8 @@ Builds a trace twin of the library (the shipped sources with -DW4A16_TRACE: lane
 %globaltimer at each phase and sums the clocks it spent waiting) next to the shipped one, runs each shape a few
 times eagerly on cuda:0 with rotating weight copies, and prints per phase the min / median / max over the CTAs of
 the last launch, relative to the first CTA's entry, plus per-role wait and work clocks per k-stage.  Reading
-%globaltimer costs a few hundred nanoseconds, so consecutive stamps of one warp are never closer than that.
+%globaltimer costs a few hundred nanoseconds, so consecutive stamps of one warp are never closer than that.  The mma.sync kernel
+(up to 8 rows, and small layers up to 16) carries no stamps: W4A16_SKINNY=0 in the environment traces the decode kernel instead.
 A debugging aid: nothing printed here is a benchmark figure, and the shipped library carries none of the stamps.
 """
 import ctypes
@@ -61,6 +62,9 @@ def run(lib, n, k, m, sms=-1, group=128, reps=5):
     full = tr.cpu().numpy().astype(np.int64)
     t, bk = full[:4096].reshape(256, 16), full[4096:].reshape(256, 16)
     used = t[:, 0] > 0
+    if not used.any():
+        print("n=%d k=%d m=%d sms=%d: the kernel of this launch carries no stamps (the mma.sync kernel?)" % (n, k, m, sms))
+        return
     t0 = t[used][:, 0].min()
     steps = np.maximum(bk[used][:, 3], 1)
     print("n=%d k=%d m=%d sms=%d: %d CTAs, %d k-stages per CTA (median)" % (n, k, m, sms, used.sum(), np.median(steps)))

@@ -44,14 +44,15 @@ extern "C" {
  *   max_par    kept for workspace sizing compatibility
  * Enqueues on `stream` and returns; 0 at once when m, n or k is 0 (marlin_cute_kernel.cu:59-60).
  * Scratch beyond the caller's workspace (fp32 partial tiles of the stream-K fix-up) is owned by the
- * library and cached per (device, stream), sized by need: the first use on a (device, stream) calls cudaMalloc
+ * library and cached per (device, stream), sized by need: the first GEMM on a (device, stream) calls cudaMalloc
  * for SMs x 64 x 128 fp32 (4.8 MB on a 148-SM B200), which covers every batch of up to 64 rows; batch tiles of
  * 128 / 192 rows grow it once to at most SMs x 192 x 128 fp32 (14.5 MB).  Growing allocates, which CUDA refuses
  * during stream capture: run a problem of each batch size once before capturing it.  A block that was outgrown
  * stays allocated (captured launches may point at it) until w4a16_release_stream.
- * Numerics: products are accumulated in fp32.  For m <= 16 with group scales the kernel accumulates the exact
- * integer weights (q - 8) per 128-k group and applies the fp16 group scale in fp32 afterwards; the reference
- * rounds (q - 8) * s to fp16 first (gemm/marlin_gemm/marlin_cute_trait.h:656-664), as this library does for larger m.
+ * Numerics: products are accumulated in fp32.  For m <= 16 with group scales and k a multiple of 256 (of 128 up to 8 rows and
+ * for some layers of 9 to 16) the kernel accumulates the exact integer weights (q - 8) per 128-k group and applies the fp16
+ * group scale in fp32 afterwards; the reference rounds (q - 8) * s to fp16 first
+ * (gemm/marlin_gemm/marlin_cute_trait.h:656-664), as this library does otherwise.
  * The two differ by that rounding only (relative 2^-11 per weight).
  * Stream order holds for A, C, workspace and the scratch.  B and s are treated as parameters: when the
  * previous kernel on `stream` is another GEMM of this library, this one may prefetch B and s while that
@@ -76,8 +77,8 @@ int w4a16_marlin_gemm(const void *A, const void *B, void *C, const void *s, int 
  * into the library (every GPU that loads the library holds it until the process exits).
  *
  * Arguments, results and return codes are those of w4a16_marlin_gemm, with these differences:
- *   - prob_m <= 64 only, and at most 160 CTAs (any sm_100 part today); beyond that it returns W4A16_ERR_ARG and
- *     w4a16_last_cuda_error() says which limit was hit.  Larger batches must use w4a16_marlin_gemm.
+ *   - prob_m <= 64 only, and as many partial tiles as the array holds (160 of 64 rows: any sm_100 part today); beyond that it
+ *     returns W4A16_ERR_ARG and w4a16_last_cuda_error() says which limit was hit.  Larger batches must use w4a16_marlin_gemm.
  *   - The first call on a device looks up the device address of the built-in array (cudaGetSymbolAddress),
  *     puts the array into its idle state on `stream` and synchronises `stream`.  Make that first call before
  *     any stream capture begins.  On EVERY call `dev` must be the current device (checked: W4A16_ERR_ARG
@@ -104,9 +105,10 @@ int w4a16_marlin_gemm_builtin_scratch(const void *A, const void *B, void *C, con
  * through the copy engines (about ten microseconds of stream time per copy, more than a decode GEMM): a small kernel
  * reads A_host over PCIe into A_stage while the GEMM behind it already prefetches its weights, and the GEMM writes its
  * result rows into C_stage and C_host.  Its copy-in may overlap the previous such calls' GEMMs on the stream where their
- * buffers do not overlap; stream order holds for all work of other origin, except a kernel that uses
- * griddepcontrol.launch_dependents before it has finished with A_host or A_stage.  Calls that alternate between streams
- * keep the copy engines, which overlap one stream's copies with another's kernels.  W4A16_HOST_DIRECT=0 in the environment
+ * buffers do not overlap (an overlap of any buffers is seen, whichever thread made the calls); stream order holds for all
+ * work of other origin, graph launches included, except a kernel that uses griddepcontrol.launch_dependents before it has
+ * finished with A_host or A_stage.  Calls that alternate between streams keep the copy engines, which overlap one stream's
+ * copies with another's kernels.  Calls may be captured; the first one of a capture waits for what is before it.  W4A16_HOST_DIRECT=0 in the environment
  * always takes the copy engines, =1 never.
  */
 int w4a16_marlin_gemm_host(const void *A_host, const void *B, void *C_host, const void *s, int prob_m, int prob_n,
@@ -197,8 +199,8 @@ const char *w4a16_plan_kernel(int prob_m, int prob_n, int prob_k, int groupsize,
 int w4a16_release_stream(int dev, void *stream);
 
 /* Self-test of the bounded device-side waits (the reference has none: its fix-up spin is unbounded,
- * include/barrier.h:85-96).  Launches the GEMM so that one CTA waits for a partial tile that no CTA will ever
- * write; after limit_ms (1..5000) the kernel gives up, unwinds and returns.  The call itself returns W4A16_OK;
+ * include/barrier.h:85-96).  Launches the GEMM, in the stream-K form of the kernel that serves its size on single CTAs, so
+ * that one CTA waits for a partial tile that no CTA will ever write; after limit_ms (1..5000) the kernel gives up, unwinds and returns.  The call itself returns W4A16_OK;
  * w4a16_device_status(dev, stream) then returns W4A16_ERR_TIMEOUT and restores the scratch, after which the
  * stream is usable as before.  C is left undefined.  Injects no GPU fault.  A negative limit_ms runs the same on the
  * built-in array of w4a16_marlin_gemm_builtin_scratch (prob_m <= 64) for -limit_ms milliseconds. */
