@@ -6,14 +6,27 @@
 //   * CTA r of the pair owns weight columns [256 T + 128 r, +128): it streams, dequantises and keeps them in ITS
 //     tensor memory, and holds ITS 128 accumulator rows;
 //   * CTA r loads only rows [m0 + r TM/2, +TM/2) of the activation tile: the UMMA (M = 256, N = TM) reads the B
-//     operand half from each CTA's shared memory.  Per CTA a 128-k stage is 8 KB of weights + TM x 128 B of
-//     activations instead of + TM x 256 B: the single-CTA kernel is bound by bytes in flight (all of shared memory
-//     holds only 4 stages of a 192-row tile); here 6 stages fit;
+//     operand half from each CTA's shared memory, so that per CTA a 128-k stage is 8 KB of weights + TM x 128 B of
+//     activations instead of + TM x 256 B;
 //   * the leader (cluster rank 0) issues every MMA; completion is signalled to both CTAs with one commit.
 // Barriers the leader's MMA warp waits on live in the leader: the partner's dequant and epilogue warps arrive on
 // them through the cluster address space, and the partner's activation loads count their bytes there.
-// Everything else (roles, stream-K with sentinel slots, bounded waits, dependent launch) is as in the single-CTA
-// kernel.  The reference has no counterpart (it is an sm_80 kernel, gemm/marlin_gemm/marlin_cute_trait.h).
+//
+// What sets the pace differs by the tile.  192 rows: the MMAs (768 clocks a 128-k stage, all of it busy) and the part's power.
+// 128 rows: the MMAs again (517 clocks), if everything around them keeps up; up to 64 rows: the conversion, 13 instructions a
+// packed word whose pipes take about 20 clocks (fp16x2 and logic operations two clocks each), 650 a 256-k stage, beside HBM
+// (700 where the whole chip streams).  Below 192 rows it was the issuer's own chain of waits (see there), hence:
+//   * one elected lane issues, and asks for the next stage's barriers before it issues this one's MMAs;
+//   * weights (with their scales) and activations have rings and producers of their own: a weight slot is free when it is
+//     converted, in a common one it would wait for the MMAs; one commit per stage frees its activations and its operand buffer;
+//   * a packed word is converted by the thread that loaded it (as in w4a16_kernel_decode.cuh), by three sets of warps up to 64 rows;
+//   * the dequant warps share the end of the CTA's last tile.
+// us in a chain of launches, weights from HBM, before -> after: 24 x 4096 x 4096 7.1 -> 6.0, 48 x 4096 x 4096 7.4 -> 6.6, 48 x 18944 x
+// 8192 25.7 -> 21.7, 32 x 22016 x 4096 18.1 -> 17.3, 77 x 5120 x 5504 11.4 -> 9.6, 128 x 8192 x 28672 55.3 -> 51.1, 256 x 8192 x 8192
+// 34.7 -> 28.0, 1024 x 4096 x 11008 73.7 -> 71.7.
+//
+// Everything else (stream-K with sentinel slots, bounded waits, dependent launch) is as in the single-CTA kernel.  The
+// reference has no counterpart (it is an sm_80 kernel, gemm/marlin_gemm/marlin_cute_trait.h).
 #pragma once
 #include "w4a16_kernel.cuh"
 
@@ -31,13 +44,11 @@ struct Config2 {
   static constexpr int W_BYTES = KS * TILE_N / 2;            // 8 or 16 KB
   static constexpr int A_BYTES = HALF_ROWS * KS * 2;         // [KS/64 chunks][TM/2 rows][128 B]
   static constexpr int S_BYTES = GROUPS * TILE_N * 2;
-  static constexpr int STAGE_BYTES = W_BYTES + A_BYTES + S_BYTES;
   static constexpr int ACC_STRIDE = TM;
   static constexpr int WBUF_COL0 = 2 * ACC_STRIDE;
   static constexpr int WBUF_COLS = KS / 2;
   static constexpr int TMEM_COLS = 512;
-  static constexpr int WBUFS_RAW = (TMEM_COLS - WBUF_COL0) / WBUF_COLS;
-  static constexpr int WBUFS = WBUFS_RAW > 4 ? 4 : WBUFS_RAW;
+  static constexpr int WBUFS = (TMEM_COLS - WBUF_COL0) / WBUF_COLS > 4 ? 4 : (TMEM_COLS - WBUF_COL0) / WBUF_COLS;
   static_assert(WBUFS >= 2, "TMEM budget");
   static constexpr int BAR_BYTES = 1024;
   static constexpr int GATHER_BYTES = staged_output(OUT) ? GATHER_SLAB_BYTES : 0;
@@ -45,20 +56,33 @@ struct Config2 {
   // cluster form: the other pairs' partial sums of the 16-row chunks this pair finishes, [chunk / P][P - 1][16][128] fp32
   static constexpr int CHUNKS = TM / 16;
   static constexpr int XSLAB_BYTES = P > 1 ? (CHUNKS + P - 1) / P * (P - 1) * 16 * TILE_N * 4 : 0;
-  static constexpr int STAGES_RAW = (SMEM_MAX - BAR_BYTES - GATHER_BYTES - XSLAB_BYTES - 1024) / STAGE_BYTES;
-  static constexpr int STAGES = STAGES_RAW > 8 ? 8 : STAGES_RAW & ~1;   // even: a stage is always converted by the same set
-  static_assert(STAGES >= 3, "ring too shallow");
-  static constexpr int NSETS = 2, NDQ = 8;
-  static constexpr int THREADS = (NDQ + EPI_WARPS + 2) * 32;
-  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + BAR_BYTES + GATHER_BYTES + XSLAB_BYTES + 1024;
+  // Two dequant sets keep ahead of the MMAs of 128 and 192 rows and leave a thread 128 registers; below, where the conversion
+  // sets the pace, three (128 rows, 2 / 3 sets, us: 77 x 5120 x 5504 9.6 / 9.3, 128 x 8192 x 28672 51.1 / 50.3, 256 x 8192 x 8192
+  // 28.0 / 29.0, 128 x 22016 x 4096 23.4-26.3 / 28.8-29.9).
+  static constexpr int NSETS = TM >= 128 ? 2 : 3, NDQ = 4 * NSETS;
+  // Activations: slots for a load's latency and the MMAs in flight; the rest of shared memory is for weights.
+  static constexpr int RINGS = SMEM_MAX - BAR_BYTES - GATHER_BYTES - XSLAB_BYTES - 1024;
+  static constexpr int A_SLOTS = TM == 32 ? 6 : TM == 64 ? 5 : TM == 128 ? (P > 2 ? 6 : 7) : P > 1 ? 4 : 6;
+  static constexpr int W_SLOTS_RAW = (RINGS - A_SLOTS * A_BYTES) / (W_BYTES + S_BYTES);
+  static constexpr int W_SLOTS = W_SLOTS_RAW > 12 ? 12 : W_SLOTS_RAW;
+  static constexpr int STAGES = W_SLOTS;
+  // A parity wait is right only for a waiter that knows the barrier's phase before the awaited one to be over.  Coming to stage
+  // g, a dequant set knows through its own stage g - NSETS that the MMAs of g - NSETS - WBUFS, and of all stages before (they
+  // complete in order), are over: their weights had landed (where the sets do not come back to their own slots the weight ring
+  // has to be that deep), and done[] of g - WBUFS - A_SLOTS is over; its next phase, of g - WBUFS + A_SLOTS, comes after g.
+  static_assert(W_SLOTS % NSETS == 0 || W_SLOTS >= NSETS + WBUFS, "no wait may pass on an older phase of its barrier");
+  static_assert(A_SLOTS >= NSETS && A_SLOTS >= WBUFS, "no wait may pass on an older phase, or miss one");
+  static constexpr int THREADS = (NDQ + EPI_WARPS + 3) * 32;
+  static constexpr int SMEM_BYTES = W_SLOTS * (W_BYTES + S_BYTES) + A_SLOTS * A_BYTES + BAR_BYTES + GATHER_BYTES + XSLAB_BYTES + 1024;
+  static_assert(SMEM_BYTES <= SMEM_MAX, "shared memory budget");
 };
 
 struct Bars2 {  // same offsets in both CTAs of the pair
-  uint64_t wsfull[8];    // weights + scales of a stage landed in THIS CTA                    (local)
+  uint64_t wsfull[12];   // a slot's weights + scales landed in THIS CTA                      (local)
+  uint64_t wfree[12];    // ... converted by its four dequant warps                           (local)
   uint64_t afull[8];     // both halves of the activation tile landed                         (used in the leader)
-  uint64_t empty[8];     // stage free again: this CTA's dequant warps + the pair's MMA commit (local)
+  uint64_t done[8];      // a stage's MMAs have completed (commit to both CTAs): its activations and operand buffer are free (local)
   uint64_t wfull[4];     // TMEM operand buffer written in both CTAs                          (used in the leader)
-  uint64_t wempty[4];    // ... read by the MMAs (commit to both CTAs)                        (local)
   uint64_t accfull[2];   // accumulator complete (commit to both CTAs)                        (local)
   uint64_t accempty[2];  // accumulator drained by both CTAs' epilogue warps                  (used in the leader)
   uint64_t drain;
@@ -139,21 +163,22 @@ w4a16_tc2_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant_
   using Cfg = Config2<TM, KS_, OUT, P>;
   constexpr bool GATHER = OUT == OUT_GATHER;
   using namespace sm100;
-  constexpr int S = Cfg::STAGES, NDQ = Cfg::NDQ, KS = Cfg::KS;
-  constexpr int PRODUCER_WARP = NDQ + EPI_WARPS, MMA_WARP = NDQ + EPI_WARPS + 1;
-  constexpr bool HELP = TM >= 64 && !staged_output(OUT);   // dequant warps help to finish a split tile (as in the single-CTA kernel)
+  constexpr int SW = Cfg::W_SLOTS, SA = Cfg::A_SLOTS, NDQ = Cfg::NDQ, KS = Cfg::KS;
+  constexpr int W_WARP = NDQ + EPI_WARPS, A_WARP = W_WARP + 1, MMA_WARP = W_WARP + 2;
+  constexpr bool HELP = !staged_output(OUT);   // the dequant warps, idle by then, share the end of the CTA's last tile
   constexpr uint32_t WS_TX = Cfg::W_BYTES + (GROUPED ? Cfg::S_BYTES : 0);
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t *sW = smem;
-  uint8_t *sA = sW + S * Cfg::W_BYTES;
-  uint8_t *sS = sA + S * Cfg::A_BYTES;
-  Bars2 *bars = reinterpret_cast<Bars2 *>(sS + S * Cfg::S_BYTES);
+  uint8_t *sA = sW + SW * Cfg::W_BYTES;
+  uint8_t *sS = sA + SA * Cfg::A_BYTES;
+  Bars2 *bars = reinterpret_cast<Bars2 *>(sS + SW * Cfg::S_BYTES);
   volatile int *abort = &bars->abort;
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
+  if (warp == 0) W4A16_STAMP(0);   // kernel entry
   const uint32_t crank = cluster_ctarank();
   const uint32_t rank = P == 1 ? crank : crank & 1;        // in the pair (0 = leader)
   const uint32_t leader = P == 1 ? 0 : crank & ~1u;        // cluster rank of the leader
@@ -184,16 +209,20 @@ w4a16_tc2_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant_
   };
 
   // ---- prologue
-  if (warp == PRODUCER_WARP && lane == 0) {
-    for (int i = 0; i < S; ++i) {
+  if (warp == W_WARP && lane == 0) {
+    for (int i = 0; i < SW; ++i) {
       mbar_init(smem_u32(&bars->wsfull[i]), 1);
+      mbar_init(smem_u32(&bars->wfree[i]), 4);
+    }
+    mbar_fence_init();
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  if (warp == A_WARP && lane == 0) {
+    for (int i = 0; i < SA; ++i) {
       mbar_init(smem_u32(&bars->afull[i]), 1);
-      mbar_init(smem_u32(&bars->empty[i]), 4 + 1);
+      mbar_init(smem_u32(&bars->done[i]), 1);
     }
-    for (int i = 0; i < Cfg::WBUFS; ++i) {
-      mbar_init(smem_u32(&bars->wfull[i]), 8);       // four dequant warps of each CTA
-      mbar_init(smem_u32(&bars->wempty[i]), 1);
-    }
+    for (int i = 0; i < Cfg::WBUFS; ++i) mbar_init(smem_u32(&bars->wfull[i]), 8);   // four dequant warps of each CTA
     for (int i = 0; i < 2; ++i) {
       mbar_init(smem_u32(&bars->accfull[i]), 1);
       mbar_init(smem_u32(&bars->accempty[i]), 2 * EPI_WARPS);
@@ -219,6 +248,7 @@ w4a16_tc2_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant_
   cluster_sync_all();              // both CTAs' barriers exist before anything can arrive on them
   tc_fence_after();
   const uint32_t tmem = __shfl_sync(0xffffffffu, bars->tmem_base, 0);
+  if (warp == 0) W4A16_STAMP(1);   // prologue done
 
   // Cluster form: this warp's part of the exchange and of the finished chunks; h of H warps per TMEM lane quadrant
   auto exchange = [&](int h, int H) {
@@ -235,6 +265,7 @@ w4a16_tc2_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant_
     const bool ok = warp_wait(smem_u32(&bars->accfull[0]), 0, abort, p.wait_ns);
     if (!ok) give_up(p, abort, 13);
     tc_fence_after();
+    if (warp == NDQ) W4A16_STAMP(6);
     const uint32_t t_acc = tmem + ((uint32_t)(quad * 32) << 16);
     float *slab = reinterpret_cast<float *>(reinterpret_cast<uint8_t *>(bars) + Cfg::BAR_BYTES + Cfg::GATHER_BYTES);
     const uint32_t slab_u = smem_u32(slab) + (uint32_t)row * 4, bar_u = smem_u32(&bars->xfull);
@@ -254,6 +285,7 @@ w4a16_tc2_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant_
     // (longer than any other wait: nothing may arrive in a CTA that has left)
     if (q * 16 < width && !warp_wait_cluster(bar_u, 0, 8 * p.wait_ns)) { give_up(p, abort, 14); return; }
     if (!ok) return;
+    if (warp == NDQ) W4A16_STAMP(7);   // the other pairs' sums arrived
 #pragma unroll 1
     for (int c = h; c * 16 < width; c += H) {
       if (c % P != q) continue;
@@ -286,84 +318,98 @@ w4a16_tc2_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant_
     }
   };
 
+  // (Three dequant sets leave a thread 96 registers, and two slices in flight would spill 80 bytes of the hot loops.  One other
+  // pair, the usual case: one slice, inline; more: two at a time in a call, which keeps them out of these registers.)
+  auto fold_slices = [&](uint32_t (&v)[16], uint32_t *partials, int rows, int c0, int row, int first_slot, int slot_stride, int count,
+                         volatile int *abort_, uint64_t t0, uint64_t wait_ns) {
+    if constexpr (Cfg::NSETS == 2) return fold_partial_slices<2>(v, partials, rows, c0, row, first_slot, slot_stride, count, abort_, t0, wait_ns);
+    if (count == 1) return fold_partial_slices<1>(v, partials, rows, c0, row, first_slot, slot_stride, 1, abort_, t0, wait_ns);
+    return fold_partial_slices_call<2>(v, partials, rows, c0, row, first_slot, slot_stride, count, abort_, t0, wait_ns);
+  };
+
   if (warp < NDQ) {
-    // =========================================================== dequant warps (as in the single-CTA kernel)
+    // =========================================================== dequant warps
     const int quad = warp & 3, set = warp >> 2;
     const int row = quad * 32 + lane;
-    const int nr = row & 63, blk = row >> 6;
-    const int j = nr >> 4, r8 = nr & 7;
-    const uint32_t shift = ((nr >> 3) & 1) ? 8u : 0u;
-    const uint32_t base_off = (uint32_t)((4 * blk + (r8 >> 1)) * 128 + 64 * ((r8 & 1) ^ blk) + 4 * j);
-    uint32_t toff[4];
-#pragma unroll
-    for (int t = 0; t < 4; ++t) toff[t] = base_off + 16u * (uint32_t)(t ^ (r8 >> 1));
-    const uint32_t s_off = (uint32_t)(2 * (64 * blk + 8 * (nr & 7) + (nr >> 3)));
+    // This lane is fragment lane `lane` of 64-column block quad / 2: of a 16-k row it takes the words of columns 16 j + lane / 4
+    // and + 8, j = 2 (quad % 2) and the next one (see w4a16_kernel_decode.cuh); their four group scales lie next to one another.
+    const int line = 4 * (quad >> 1) + (lane >> 3);
+    const uint32_t off = (uint32_t)(line * 128 + 16 * ((lane & 7) ^ line) + 8 * (quad & 1));
+    const uint32_t s_off = (uint32_t)(2 * (64 * (quad >> 1) + 8 * (lane >> 2) + 4 * (quad & 1)));
     const uint32_t sW_u = smem_u32(sW), sS_u = smem_u32(sS);
-    const uint32_t one2 = 0x3c003c00u;
-    const uint32_t t_lane = tmem + ((uint32_t)(quad * 32) << 16) + Cfg::WBUF_COL0;
+    const uint32_t t_dst = tmem + ((uint32_t)(quad * 32) << 16) + Cfg::WBUF_COL0;
+    const uint32_t wfull_bar = map_to_cta(smem_u32(&bars->wfull[0]), leader);
     long long d_full = 0, d_wempty = 0, d_work = 0;
     for (int g = set; g < nsteps; g += Cfg::NSETS) {
-      const int st = g % S, wb = g % Cfg::WBUFS;
+      const int st = g % SW;
       const long long c0 = W4A16_CLK();
-      if (!warp_wait(smem_u32(&bars->wsfull[st]), (g / S) & 1, abort, p.wait_ns)) { give_up(p, abort, 11); break; }
+      if (!warp_wait(smem_u32(&bars->wsfull[st]), (g / SW) & 1, abort, p.wait_ns)) { give_up(p, abort, 11); break; }
       const long long c1 = W4A16_CLK();
+      if (warp == 0 && g == 0) W4A16_STAMP(2);   // first stage landed
       d_full += c1 - c0;
-      const uint32_t wbase = sW_u + st * Cfg::W_BYTES;
-      __half2 sc = *reinterpret_cast<const __half2 *>(&one2);
-      bool buf_ok = true;
+      const uint32_t wbase = sW_u + st * Cfg::W_BYTES + off;
+      const int last = g - Cfg::WBUFS, wb = g % Cfg::WBUFS;   // the stage that had this operand buffer
+      const uint32_t last_bar = smem_u32(&bars->done[last % SA]), last_par = (last / SA) & 1;
+      bool buf_ok = last < 0 || mbar_test(last_bar, last_par);     // (needed only with the first words converted; asked for now)
 #pragma unroll
-      for (int half = 0; half < Cfg::KCHUNKS; ++half) {
-        if (GROUPED && (half & 1) == 0) {   // a new 128-k group starts every second 64-k chunk
-          uint16_t sv;
-          asm volatile("ld.shared.u16 %0, [%1];" : "=h"(sv) : "r"(sS_u + st * Cfg::S_BYTES + (half >> 1) * (TILE_N * 2) + s_off));
-          sc = __half2half2(__ushort_as_half(sv));
-        }
-        uint32_t v[32];
+      for (int h = 0; h < Cfg::GROUPS; ++h) {    // 128-k groups
+        uint32_t wx[8], wy[8], s01 = 0, s23 = 0;
+        if (GROUPED) asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(s01), "=r"(s23) : "r"(sS_u + st * Cfg::S_BYTES + h * (TILE_N * 2) + s_off));
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
+        for (int rr = 0; rr < 8; ++rr)
+          asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(wx[rr]), "=r"(wy[rr]) : "r"(wbase + (h * 8 + rr) * 1024));
 #pragma unroll
-          for (int t = 0; t < 4; ++t) {
-            uint32_t w;
-            asm volatile("ld.shared.u32 %0, [%1];" : "=r"(w) : "r"(wbase + (half * 4 + r) * 1024 + toff[t]));
-            dequant_word<GROUPED>(w >> shift, sc, v[r * 8 + t], v[r * 8 + 4 + t]);
+        for (int jj = 0; jj < 2; ++jj) {         // the two 16-column groups of this quadrant
+          const uint32_t s2 = jj ? s23 : s01;
+          const __half2 sc = *reinterpret_cast<const __half2 *>(&s2), lo = __low2half2(sc), hi = __high2half2(sc);
+          uint32_t v[32];
+#pragma unroll
+          for (int rr = 0; rr < 8; ++rr) {
+            const uint32_t w = jj ? wy[rr] : wx[rr];
+            // registers (4 rr, +1, +2, +3) = (column n, k-pair t), (n + 8, t), (n, t + 4), (n + 8, t + 4) of 16-k row rr
+            dequant_word<GROUPED>(w, lo, v[4 * rr], v[4 * rr + 2]);
+            dequant_word<GROUPED>(w >> 8, hi, v[4 * rr + 1], v[4 * rr + 3]);
           }
+          if (h == 0 && jj == 0) {
+            const long long c2 = W4A16_CLK();
+            if (!__all_sync(0xffffffffu, buf_ok)) buf_ok = warp_wait(last_bar, last_par, abort, p.wait_ns);
+            tc_fence_after();
+            d_wempty += W4A16_CLK() - c2;
+            if (!buf_ok) break;
+          }
+          tmem_st_16x128b_x16(t_dst + wb * Cfg::WBUF_COLS + ((uint32_t)(16 * jj) << 16) + h * 64, v);
         }
-        if (half == 0) {
-          const long long c2 = W4A16_CLK();
-          buf_ok = warp_wait(smem_u32(&bars->wempty[wb]), ((g / Cfg::WBUFS) & 1) ^ 1, abort, p.wait_ns);
-          tc_fence_after();
-          d_wempty += W4A16_CLK() - c2;
-          if (!buf_ok) break;
-        }
-        tmem_st_32x32b_x32(t_lane + wb * Cfg::WBUF_COLS + half * 32, v);
+        if (!buf_ok) break;
       }
       if (!buf_ok) { give_up(p, abort, 12); break; }
       tc_wait_st();
       tc_fence_before();
       __syncwarp();
       if (lane == 0) {
-        mbar_arrive_cluster(map_to_cta(smem_u32(&bars->wfull[wb]), leader));   // the leader's MMA warp counts both CTAs
-        mbar_arrive(smem_u32(&bars->empty[st]));
+        mbar_arrive_cluster(wfull_bar + 8 * wb);   // the leader's MMA warp counts both CTAs
+        mbar_arrive(smem_u32(&bars->wfree[st]));
       }
       d_work += W4A16_CLK() - c1;
+      if (warp == 0 && g == 0) W4A16_STAMP(3);   // first operand tile in TMEM
     }
+    if (warp == 0) W4A16_STAMP(4);   // last dequant of set 0
     if (warp == 0) { W4A16_BUCKET(4, d_full); W4A16_BUCKET(5, d_wempty); W4A16_BUCKET(6, d_work); }
     if (P > 1) {
-      if (HELP) exchange(1 + set, 1 + Cfg::NSETS);
+      exchange(1 + set, 1 + Cfg::NSETS);
     } else if (HELP) {
-      // ---- help to finish the CTA's last tile if it is a split one (chunks 16*(1+set), +48, ... of this quadrant)
+      // ---- help to finish the CTA's last tile if it is this pair's to finish (chunks 1 + set, 1 + set + (1 + NSETS), ... of this quadrant)
       int l_tile = 0, l_kb = 1, l_ke = 0, l_seg = -1;
       {
         Walk<P> walk(p, pair);
         int t, kb, ke;
         while (walk.next(t, kb, ke)) l_tile = t, l_kb = kb, l_ke = ke, ++l_seg;
       }
-      if (l_seg >= 0 && l_kb == 0 && l_ke < p.k_iters) {
+      if (l_seg >= 0 && l_kb == 0) {
         int l_n, l_m;
         tile_nm(p, l_tile, l_n, l_m);
         const int n0 = (2 * l_n + (int)rank) * TILE_N, m0 = l_m * TM;
         const int acc = l_seg & 1;
-        const int last_pair = ((l_tile - p.sk_tile0 + 1) * p.k_iters - 1) / p.iters_per_cta;
+        const int ncontrib = l_ke < p.k_iters ? ((l_tile - p.sk_tile0 + 1) * p.k_iters - 1) / p.iters_per_cta - pair : 0;
         __half sch = __float2half(1.0f);
         if (!GROUPED) {
           const int c32 = row & 31;
@@ -376,12 +422,12 @@ w4a16_tc2_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant_
         const uint32_t t_acc = tmem + ((uint32_t)(quad * 32) << 16) + acc * Cfg::ACC_STRIDE;
         const int width = tile_width<TM>(p, m0);
 #pragma unroll 1
-        for (int c0 = 16 * (1 + set); c0 < width && ok; c0 += 48) {
+        for (int c0 = 16 * (1 + set); c0 < width && ok; c0 += 16 * (1 + Cfg::NSETS)) {
           uint32_t v[16];
           tmem_ld_32x32b_x16(t_acc + c0, v);
           tc_wait_ld();
           // contributors are the same-rank CTAs of the following pairs: slots 2 (pair + 1) + rank, + 2, ...
-          ok = fold_partial_slices<2>(v, p.partials, TM, c0, row, 2 * (pair + 1) + (int)rank, 2, last_pair - pair, abort, t0, p.wait_ns);
+          if (ncontrib > 0) ok = fold_slices(v, p.partials, TM, c0, row, 2 * (pair + 1) + (int)rank, 2, ncontrib, abort, t0, p.wait_ns);
           if (!ok) break;
 #pragma unroll
           for (int i = 0; i < 16; ++i) {   // (never the gathering form: HELP is off there)
@@ -395,7 +441,7 @@ w4a16_tc2_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant_
       }
     }
   } else if (P > 1 && warp < NDQ + EPI_WARPS) {
-    exchange(0, HELP ? 1 + Cfg::NSETS : 1);
+    exchange(0, 1 + Cfg::NSETS);
   } else if (warp < NDQ + EPI_WARPS) {
     // =========================================================== epilogue warps: this CTA's 128 columns, all TM rows
     const int quad = warp & 3;
@@ -405,13 +451,14 @@ w4a16_tc2_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant_
     __half *slabs = reinterpret_cast<__half *>(reinterpret_cast<uint8_t *>(bars) + Cfg::BAR_BYTES);   // gathering form only
     int gcount = 0;
     Walk<P> walk(p, pair);
-    int tile, kb, ke;
+    int tile, kb, ke, left = nsteps;
     for (int seg = 0; walk.next(tile, kb, ke); ++seg) {
       int n_idx2, m_idx;
       tile_nm(p, tile, n_idx2, m_idx);
       const int n0 = (2 * n_idx2 + (int)rank) * TILE_N, m0 = m_idx * TM;
       const int acc = seg & 1;
       const bool finisher = (kb == 0);
+      left -= ke - kb;
       // contributors are the same-rank CTAs of the following pairs: slots blockIdx.x + 2, + 4, ...
       const int last_pair = (finisher && ke < p.k_iters) ? ((tile - p.sk_tile0 + 1) * p.k_iters - 1) / p.iters_per_cta : pair;
       const int ncontrib = last_pair - pair;
@@ -422,11 +469,12 @@ w4a16_tc2_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant_
       }
       if (!warp_wait(smem_u32(&bars->accfull[acc]), (seg >> 1) & 1, abort, p.wait_ns)) { give_up(p, abort, 13); break; }
       tc_fence_after();
+      if (warp == NDQ && seg == 0) W4A16_STAMP(5);   // first accumulator complete
+      if (warp == NDQ) W4A16_STAMP(6);               // (last value wins) last accumulator complete
       uint32_t *part = p.partials + ((size_t)blockIdx.x * TM) * TILE_N + row;
       bool ok = true;
       const uint64_t t0 = ncontrib > 0 ? globaltimer_ns() : 0ull;
-      constexpr int FLY = 2;
-      const int c_step = (HELP && finisher && ncontrib > 0) ? 48 : 16;   // the dequant warps take the other chunks
+      const int c_step = (HELP && finisher && left == 0) ? 16 * (1 + Cfg::NSETS) : 16;   // the dequant warps take the other chunks
       const int width = tile_width<TM>(p, m0);
 #pragma unroll 1
       for (int c0 = 0; c0 < width && ok; c0 += c_step) {
@@ -437,7 +485,7 @@ w4a16_tc2_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant_
 #pragma unroll
           for (int i = 0; i < 16; ++i) st_slot(part + (size_t)(c0 + i) * TILE_N, v[i] == PARTIAL_IDLE ? 0x7fffffffu : v[i]);
         } else {
-          if (ncontrib > 0) ok = fold_partial_slices<FLY>(v, p.partials, TM, c0, row, 2 * (pair + 1) + (int)rank, 2, ncontrib, abort, t0, p.wait_ns);
+          if (ncontrib > 0) ok = fold_slices(v, p.partials, TM, c0, row, 2 * (pair + 1) + (int)rank, 2, ncontrib, abort, t0, p.wait_ns);
           if (!ok) break;
           if constexpr (GATHER) {
             if (!store_chunk_gather4<GROUPED>(p, v, sch, m0 + c0, n0, quad, lane, slabs, smem_u32(&bars->gfull[0]), gcount, abort)) {
@@ -461,6 +509,7 @@ w4a16_tc2_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant_
         }
       }
       if (!ok) { give_up(p, abort, 14); break; }
+      if (warp == NDQ) W4A16_STAMP(8);               // (last value wins) epilogue done
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&bars->accempty[acc]), leader));
@@ -468,120 +517,145 @@ w4a16_tc2_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant_
     // the TMA stores of this thread have left shared memory and reached C before the CTA ends (also after a give-up)
     if (OUT == OUT_TMA && quad == 0 && lane == 0) tma_store_wait_all();
     if (OUT == OUT_GATHER) tma_store_wait_all();   // every lane issues row copies in the gathering form
-  } else if (warp == PRODUCER_WARP) {
-    // =========================================================== TMA producer (one per CTA, each for its own halves)
-    const int first = min(S, nsteps);
+  } else if (warp == W_WARP) {
+    // =========================================================== TMA producer of weights and scales: parameters, so they are
+    // requested (and converted) while the previous kernel of the stream may still run
     int step = 0;
-    {  // weights of the first ring-full: parameters, requested before the previous kernel of the stream is known done
-      Walk<P> walk(p, pair);
-      int tile, kb, ke, i = 0;
-      while (i < first && walk.next(tile, kb, ke)) {
-        int n_idx2, m_idx;
-        tile_nm(p, tile, n_idx2, m_idx);
-        for (int kk = kb; kk < ke && i < first; ++kk, ++i) {
-          if (elect_one()) issue_weights(i, n_idx2, kk);
-          __syncwarp();
+    bool ok = true, told = false;
+    long long c_wait = 0, c_issue = 0;
+    Walk<P> walk(p, pair);
+    int tile, kb, ke;
+    while (ok && walk.next(tile, kb, ke)) {
+      int n_idx2, m_idx;
+      tile_nm(p, tile, n_idx2, m_idx);
+      for (int kk = kb; kk < ke; ++kk, ++step) {
+        const int st = step % SW;
+        if (step >= SW) {
+          if (!told) pdl_launch_dependents(), told = true;
+          const long long c0 = W4A16_CLK();
+          if (!warp_wait(smem_u32(&bars->wfree[st]), ((step / SW) & 1) ^ 1, abort, p.wait_ns)) { give_up(p, abort, 15); ok = false; break; }
+          c_wait += W4A16_CLK() - c0;
         }
+        const long long c1 = W4A16_CLK();
+        if (elect_one()) issue_weights(st, n_idx2, kk);
+        __syncwarp();
+        c_issue += W4A16_CLK() - c1;
       }
     }
-    pdl_launch_dependents();
-    pdl_wait_prior_grid();
-    {
-      Walk<P> walk(p, pair);
-      int tile, kb, ke;
-      bool ok = !__any_sync(0xffffffffu, *abort);   // (given up while the previous kernel ran: nothing new into a CTA that ends)
-      while (ok && walk.next(tile, kb, ke)) {
-        int n_idx2, m_idx;
-        tile_nm(p, tile, n_idx2, m_idx);
-        const int m0 = m_idx * TM;
-        for (int kk = kb; kk < ke; ++kk, ++step) {
-          const int st = step % S;
-          if (step >= first) {
-            if (!warp_wait(smem_u32(&bars->empty[st]), ((step / S) & 1) ^ 1, abort, p.wait_ns)) { give_up(p, abort, 15); ok = false; break; }
-          }
-          if (elect_one()) {
-            if (step >= first) issue_weights(st, n_idx2, kk);
-            issue_acts(st, m0, kk);
-          }
-          __syncwarp();
-        }
-      }
-    }
+    if (!told) pdl_launch_dependents();
+    W4A16_STAMP(10);   // last weights requested
+    W4A16_BUCKET(0, c_wait); W4A16_BUCKET(1, c_issue);
     if (*abort) {   // unwinding: let the copies in flight land
       volatile int never = 0;
-      const int issued = max(step, first);
-      for (int i = max(0, issued - S); i < issued; ++i) mbar_wait(smem_u32(&bars->wsfull[i % S]), (i / S) & 1, &never, 200000000ull);
-      if (rank == 0) {
-        // Both CTAs' activation bytes are counted here, and the CTAs leave together.  (200 ms in all: a partner that gave up
-        // before this one has not requested all of these stages.)
-        const uint64_t t0 = globaltimer_ns(), most = 200000000ull;
-        for (int i = max(0, step - S); i < step; ++i) {
-          const uint64_t spent = globaltimer_ns() - t0;
-          mbar_wait(smem_u32(&bars->afull[i % S]), (i / S) & 1, &never, spent < most ? most - spent : 1);
+      for (int i = max(0, step - SW); i < step; ++i) mbar_wait(smem_u32(&bars->wsfull[i % SW]), (i / SW) & 1, &never, 200000000ull);
+    }
+  } else if (warp == A_WARP) {
+    // =========================================================== TMA producer of activations (one per CTA, each its own half)
+    pdl_wait_prior_grid();
+    int step = 0;
+    Walk<P> walk(p, pair);
+    int tile, kb, ke;
+    bool ok = !__any_sync(0xffffffffu, *abort);   // (given up while the previous kernel ran: nothing new into a CTA that ends)
+    while (ok && walk.next(tile, kb, ke)) {
+      int n_idx2, m_idx;
+      tile_nm(p, tile, n_idx2, m_idx);
+      const int m0 = m_idx * TM;
+      for (int kk = kb; kk < ke; ++kk, ++step) {
+        const int st = step % SA;
+        if (step >= SA) {
+          if (!warp_wait(smem_u32(&bars->done[st]), ((step / SA) & 1) ^ 1, abort, p.wait_ns)) { give_up(p, abort, 7); ok = false; break; }
         }
+        if (elect_one()) issue_acts(st, m0, kk);
+        __syncwarp();
+      }
+    }
+    if (*abort && rank == 0) {   // unwinding: let the copies in flight land
+      // Both CTAs' activation bytes are counted here, and the CTAs leave together.  (200 ms in all: a partner that gave up
+      // before this one has not requested all of these stages.)
+      volatile int never = 0;
+      const uint64_t t0 = globaltimer_ns(), most = 200000000ull;
+      for (int i = max(0, step - SA); i < step; ++i) {
+        const uint64_t spent = globaltimer_ns() - t0;
+        mbar_wait(smem_u32(&bars->afull[i % SA]), (i / SA) & 1, &never, spent < most ? most - spent : 1);
       }
     }
   } else if (rank == 0) {
-    // =========================================================== MMA issuer: the leader's warp, for both CTAs
-    int step = 0, seg = 0;
+    // =========================================================== MMA issuer: one lane of the leader's warp, for both CTAs
+    // One elected lane runs the whole loop, and asks for the next stage before it issues this one's MMAs: a wait whose
+    // barrier is ready costs a warp about 200 clocks (with the vote, and one after the other), eight MMAs and a commit 90, so
+    // that a stage took 520 to 600 clocks to issue where its MMAs run for 264 (64 rows) or 517 (128).  This way 290 to 340.
     bool ok = true;
     long long m_afull = 0, m_wfull = 0, m_issue = 0, m_acc = 0;
-    const uint32_t sA_u = smem_u32(sA);
-    const uint16_t pair_mask = P == 1 ? 3 : (uint16_t)(3u << leader);
-    Walk<P> walk(p, pair);
-    int tile, kb, ke;
-    for (; ok && walk.next(tile, kb, ke); ++seg) {
-      int n_idx2, m_idx;
-      tile_nm(p, tile, n_idx2, m_idx);
-      const uint32_t idesc = make_idesc_f16_f32(2 * TILE_N, tile_width<TM>(p, m_idx * TM));   // UMMA N = the tile's own rows
-      const int acc = seg & 1;
-      const long long ca = W4A16_CLK();
-      if (!warp_wait(smem_u32(&bars->accempty[acc]), ((seg >> 1) & 1) ^ 1, abort, p.wait_ns)) { give_up(p, abort, 16); ok = false; break; }
-      m_acc += W4A16_CLK() - ca;
-      const uint32_t d_tmem = tmem + acc * Cfg::ACC_STRIDE;
-      for (int kk = kb; kk < ke && ok; ++kk, ++step) {
-        const int st = step % S, wb = step % Cfg::WBUFS;
-        const long long c0 = W4A16_CLK();
-        if (!warp_wait(smem_u32(&bars->afull[st]), (step / S) & 1, abort, p.wait_ns)) { give_up(p, abort, 17); ok = false; break; }
-        const long long c1 = W4A16_CLK();
-        if (!warp_wait(smem_u32(&bars->wfull[wb]), (step / Cfg::WBUFS) & 1, abort, p.wait_ns)) { give_up(p, abort, 18); ok = false; break; }
-        tc_fence_after();
-        const long long c2 = W4A16_CLK();
-        m_afull += c1 - c0;
-        m_wfull += c2 - c1;
-        const uint32_t a_tmem = tmem + Cfg::WBUF_COL0 + wb * Cfg::WBUF_COLS;
-        const uint64_t b_desc = make_smem_desc_sw128(sA_u + st * Cfg::A_BYTES);
-        if (elect_one()) {
+    if (elect_one()) {
+      int st = 0, wb = 0, seg = 0, step = 0;
+      uint32_t a_par = 0, w_par = 0;      // parities of the rings' current rounds
+      bool ready = false;                 // the next stage's operands are there
+      const uint32_t afull = smem_u32(&bars->afull[0]), wfull = smem_u32(&bars->wfull[0]), done = smem_u32(&bars->done[0]);
+      const uint64_t b_desc0 = make_smem_desc_sw128(smem_u32(sA));
+      const uint16_t pair_mask = P == 1 ? 3 : (uint16_t)(3u << leader);
+      Walk<P> walk(p, pair);
+      int tile, kb, ke;
+      for (; ok && walk.next(tile, kb, ke); ++seg) {
+        int n_idx2, m_idx;
+        tile_nm(p, tile, n_idx2, m_idx);
+        const uint32_t idesc = make_idesc_f16_f32(2 * TILE_N, tile_width<TM>(p, m_idx * TM));   // UMMA N = the tile's own rows
+        const int acc = seg & 1;
+        const long long ca = W4A16_CLK();
+        if (!mbar_wait(smem_u32(&bars->accempty[acc]), ((seg >> 1) & 1) ^ 1, abort, p.wait_ns)) { give_up(p, abort, 16); ok = false; break; }
+        m_acc += W4A16_CLK() - ca;
+        const uint32_t d_tmem = tmem + acc * Cfg::ACC_STRIDE;
+        for (int kk = kb; kk < ke; ++kk, ++step) {
+          const long long c0 = W4A16_CLK();
+          if (!ready) {
+            if (!mbar_wait(afull + 8 * st, a_par, abort, p.wait_ns)) { give_up(p, abort, 17); ok = false; break; }
+            const long long c1 = W4A16_CLK();
+            m_afull += c1 - c0;
+            if (!mbar_wait(wfull + 8 * wb, w_par, abort, p.wait_ns)) { give_up(p, abort, 18); ok = false; break; }
+            m_wfull += W4A16_CLK() - c1;
+          }
+          tc_fence_after();
+          const long long c2 = W4A16_CLK();
+          const uint32_t a_tmem = tmem + Cfg::WBUF_COL0 + wb * Cfg::WBUF_COLS, done_bar = done + 8 * st;
+          const uint64_t b_desc = b_desc0 + (uint64_t)(st * Cfg::A_BYTES >> 4);
+          if (++st == SA) st = 0, a_par ^= 1;
+          if (++wb == Cfg::WBUFS) wb = 0, w_par ^= 1;
+          const bool next_a = mbar_test(afull + 8 * st, a_par), next_w = mbar_test(wfull + 8 * wb, w_par);
 #pragma unroll
           for (int q = 0; q < KS / 16; ++q) {
             // per CTA the 64-k chunks are HALF_ROWS*128 bytes apart; 16 k inside a swizzle row are 32 bytes apart
             const uint64_t bd = b_desc + (uint64_t)(((q >> 2) * (Cfg::HALF_ROWS * 128) + (q & 3) * 32) >> 4);
-            tc_mma_ts_pair(d_tmem, a_tmem + q * 8, bd, idesc, (kk > kb || q > 0) ? 1u : 0u);
+            if (q == 0)
+              tc_mma_ts_pair(d_tmem, a_tmem, bd, idesc, kk > kb ? 1u : 0u);
+            else
+              tc_mma_ts_pair_imm<1>(d_tmem, a_tmem + q * 8, bd, idesc);
           }
-          tc_commit_pair(smem_u32(&bars->wempty[wb]), pair_mask);
-          tc_commit_pair(smem_u32(&bars->empty[st]), pair_mask);
+          tc_commit_pair(done_bar, pair_mask);
+          ready = next_a && next_w;
+          m_issue += W4A16_CLK() - c2;
+          if (step == 0) W4A16_STAMP(11);   // first MMA issued
         }
-        __syncwarp();
-        m_issue += W4A16_CLK() - c2;
+        if (ok) tc_commit_pair(smem_u32(&bars->accfull[acc]), pair_mask);
       }
-      if (ok && elect_one()) tc_commit_pair(smem_u32(&bars->accfull[acc]), pair_mask);
-      __syncwarp();
+      if (!ok || *abort) {   // unwinding: no MMA may still be running when tensor memory is freed
+        volatile int never = 0;
+        tc_commit_pair(smem_u32(&bars->drain), pair_mask);
+        mbar_wait(smem_u32(&bars->drain), 0, &never, 200000000ull);
+      }
+      W4A16_BUCKET(3, step);
+      W4A16_STAMP(12);   // last MMA issued
     }
-    W4A16_BUCKET(8, m_afull); W4A16_BUCKET(9, m_wfull); W4A16_BUCKET(10, m_issue); W4A16_BUCKET(11, m_acc); W4A16_BUCKET(3, step);
-    if (!ok || *abort) {   // unwinding: no MMA may still be running when tensor memory is freed
-      volatile int never = 0;
-      if (elect_one()) tc_commit_pair(smem_u32(&bars->drain), pair_mask);
-      __syncwarp();
-      mbar_wait(smem_u32(&bars->drain), 0, &never, 200000000ull);
-    }
+    __syncwarp();
+    W4A16_BUCKET(8, m_afull); W4A16_BUCKET(9, m_wfull); W4A16_BUCKET(10, m_issue); W4A16_BUCKET(11, m_acc);
   }
 
   // ---- teardown: both CTAs meet (every wait above is bounded), so that no arrive can target a CTA that has left
   tc_fence_before();
-  cluster_sync_all();
+  cluster_arrive_relaxed();
+  cluster_wait();
   if (warp == MMA_WARP) {
     tc_fence_after();
     tmem_dealloc_pair(tmem, Cfg::TMEM_COLS);
+    W4A16_STAMP(13);   // TMEM freed
   }
 }
 

@@ -1,0 +1,122 @@
+"""The barrier protocol of the CTA-pair kernel in a host model (see test_ring_waits.py): both CTAs' roles run as coroutines over
+model barriers, one copy held back as long as anything else can move.  No role may read a slot or an operand buffer that does
+not hold what is due, nobody may overwrite what is still to be read, and nobody may wait for good.  The rings are those that
+the kernel is compiled with (tests/cpp/pair_rings.cu)."""
+import os
+import random
+import subprocess
+
+import pytest
+
+import __graft_entry__ as entry
+from test_ring_waits import Bar, Stale
+
+PROGRAM = os.path.join(entry.ROOT, "tests", "cpp", "pair_rings")
+
+
+def run(c, nsteps, late, seed):
+    rng = random.Random(seed)
+    SW, SA, WB, sets = (c[x] for x in ("w_slots", "a_slots", "bufs", "sets"))
+    bars = lambda n, count: [Bar(count) for _ in range(n)]
+    both = lambda make: [make(), make()]
+    wsfull, wfree, done = both(lambda: bars(SW, 1)), both(lambda: bars(SW, 1)), both(lambda: bars(SA, 1))
+    afull, wfull = bars(SA, 2), bars(WB, 2)                       # in the leader, for both CTAs
+    slot_w, slot_a, operand = both(lambda: [None] * SW), both(lambda: [None] * SA), both(lambda: ["free"] * WB)
+    copies, mmas = [], []
+
+    def expect(have, want, what):
+        if have != want:
+            raise Stale("%s of %s where %s is due" % (what, have, want))
+
+    def weights(cta):
+        for g in range(nsteps):
+            if g >= SW:
+                yield wfree[cta][g % SW], (g // SW & 1) ^ 1
+            copies.append(("w", cta, g))
+
+    def acts(cta):
+        for g in range(nsteps):
+            if g >= SA:
+                yield done[cta][g % SA], (g // SA & 1) ^ 1
+            copies.append(("a", cta, g))
+
+    def dequant(cta, s):
+        for g in range(s, nsteps, sets):
+            yield wsfull[cta][g % SW], g // SW & 1
+            expect(slot_w[cta][g % SW], g, "weights")
+            if g >= WB:
+                yield done[cta][(g - WB) % SA], (g - WB) // SA & 1
+            expect(operand[cta][g % WB], "free", "operand buffer")
+            operand[cta][g % WB] = g
+            wfull[g % WB].arrive()
+            wfree[cta][g % SW].arrive()
+
+    def issuer():
+        for g in range(nsteps):
+            yield afull[g % SA], g // SA & 1
+            yield wfull[g % WB], g // WB & 1
+            for cta in (0, 1):
+                expect(slot_a[cta][g % SA], g, "activations")
+                expect(operand[cta][g % WB], g, "operand")
+            mmas.append(g)
+
+    def land(kind, cta, g):
+        if kind == "w":
+            slot_w[cta][g % SW] = g
+            wsfull[cta][g % SW].arrive()
+        else:
+            slot_a[cta][g % SA] = g
+            afull[g % SA].arrive()
+
+    def complete():      # in order, in both CTAs
+        g = mmas.pop(0)
+        for cta in (0, 1):
+            expect(slot_a[cta][g % SA], g, "activations")
+            operand[cta][g % WB] = "free"
+            done[cta][g % SA].arrive()
+
+    roles = [issuer()] + [r for cta in (0, 1) for r in [weights(cta), acts(cta)] + [dequant(cta, s) for s in range(sets)]]
+    waits = {r: next(r, None) for r in roles}
+    while any(w is not None for w in waits.values()):
+        moves = [("role", r) for r, w in waits.items() if w is not None and w[0].passes(w[1])]
+        moves += [("mma", None)] if mmas else []
+        moves += [("copy", x) for x in copies if x != late]
+        if not moves:
+            if late not in copies:
+                raise Stale("every role waits")
+            moves = [("copy", late)]
+        what, x = rng.choice(moves)
+        if what == "role":
+            waits[x] = next(x, None)
+        elif what == "mma":
+            complete()
+        else:
+            copies.remove(x)
+            land(*x)
+
+
+def explore(c):
+    nsteps = 2 * max(c["w_slots"], c["a_slots"]) + 3
+    for kind in "wa":
+        for g in range(nsteps):
+            for cta in (0, 1):
+                run(c, nsteps, (kind, cta, g), g)
+
+
+def test_rings_as_compiled():
+    if not os.path.exists(PROGRAM):
+        entry._make(os.path.dirname(PROGRAM))
+    out = subprocess.run([PROGRAM], capture_output=True, text=True, check=True).stdout
+    rows = [{k: int(v) for k, v in (x.split("=") for x in line.split())} for line in out.splitlines()]
+    assert len(rows) == 28
+    for c in {tuple((x, r[x]) for x in ("w_slots", "a_slots", "bufs", "sets")) for r in rows}:
+        explore(dict(c))
+
+
+@pytest.mark.parametrize("c", [
+    dict(w_slots=5, a_slots=8, bufs=4, sets=3),     # a set reads a weight slot before its data
+    dict(w_slots=8, a_slots=3, bufs=4, sets=2)])    # done[] goes round under a set that waits
+def test_the_model_sees_rings_that_are_too_small(c):
+    with pytest.raises(Stale):
+        for _ in range(4):
+            explore(c)
